@@ -200,6 +200,11 @@ nsg::PlanDesc make_plan_desc(const nsg::TopologyPlan& p, std::vector<int32_t>& p
     if (pool.capacity() < need) pool.reserve(std::max(need, 2 * pool.capacity()));
     p.append_to(pool, d.off);
     d.words = p.device_words();
+    d.lp_words = static_cast<int32_t>(p.lp.size());
+    d.lp_core = p.lp_core;
+    std::copy(p.lp_steps, p.lp_steps + 4, d.lp_steps);
+    d.lp_src = p.lp_src;
+    d.lp_perm = p.lp_perm;
     // the span [off[0], off[0] + words) may run past the last array by the
     // alignment slack: keep it inside the pool
     pool.insert(pool.end(), 4 * nsg::PA_COUNT, 0);
@@ -229,6 +234,7 @@ int intern_topology(std::vector<std::unique_ptr<nsg_topology>>& topos,
                     std::unique_ptr<nsg_topology> t) {
     for (size_t k = 0; k < topos.size(); ++k)
         if (same_plan(topos[k]->plan, t->plan)) return static_cast<int>(k);
+    nsg::build_level_program(t->plan);
     topos.push_back(std::move(t));
     return static_cast<int>(topos.size()) - 1;
 }
@@ -254,6 +260,15 @@ int32_t grid_tail_from(const nsg::TopologyPlan& p) {
     int32_t j = p.n;
     while (j > 0 && p.diag_pos[j - 1] - p.col_ptr[j - 1] >= kGridTailUpdates) --j;
     return (p.n - j >= 2) ? j : p.n;
+}
+
+PlanStage plan_stage(const std::vector<std::unique_ptr<nsg_topology>>& topos, bool transposed) {
+    PlanStage s{0, 0};
+    for (const auto& t : topos) {
+        s.doubles = std::max(s.doubles, t->plan.lp_doubles());
+        s.words = std::max(s.words, t->plan.stage_words(transposed));
+    }
+    return s;
 }
 
 void place_lu_workspace(nsg::DcDesc& d, const nsg::TopologyPlan& p, int64_t& work_size) {

@@ -19,7 +19,8 @@ cudaError_t launch_newton_dc(const PlanDesc* plans, const int32_t* lu_pool, cons
                              const double* params, double* work, double* solutions,
                              int32_t* status, int32_t* iterations, DcCtl* ctls,
                              const NewtonOptions& opt, int max_col, int max_n,
-                             long long max_stage, int32_t* rmaps, cudaStream_t stream);
+                             long long max_stage, int lp_doubles, int plan_words,
+                             int32_t* rmaps, cudaStream_t stream);
 size_t dc_smem_bytes(int max_col, int max_n);
 cudaError_t launch_dc_adjoint(const PlanDesc* plans, const int32_t* lu_pool, const DcDesc* descs,
                               int count, const int32_t* prog, const double* params, double* work,
@@ -525,6 +526,7 @@ int nsg_dc_batch_create(int count, nsg_circuit* const* circuits, int symbolic, i
                 }
             if (topo_of[i] < 0) {
                 topo_of[i] = static_cast<int>(b->topos.size());
+                nsg::build_level_program(ordered[i]->plan);
                 b->topos.push_back(std::move(ordered[i]));
             }
         }
@@ -747,13 +749,14 @@ int nsg_dc_batch_run(nsg_dc_batch* b, const double* d_params, double* d_solution
             }
         }
         int32_t* rmaps = b->row_maps ? b->d_rmap : nullptr;
+        PlanStage need = plan_stage(b->topos, false);
         auto first_launch = [&](cudaStream_t s) -> cudaError_t {
             cudaError_t r = cudaMemsetAsync(b->d_ctl, 0, sizeof(nsg::DcCtl) * b->count, s);
             if (r == cudaSuccess)
                 r = nsg::launch_newton_dc(b->d_plans, b->d_lu_pool, b->d_descs, nullptr, b->count,
                                           b->d_prog, params, b->d_work, d_solutions, d_status,
                                           d_iterations, b->d_ctl, b->opt, b->max_col, b->max_n,
-                                          max_stage_len(b->descs), rmaps, s);
+                                          max_stage_len(b->descs), need.doubles, need.words, rmaps, s);
             return r;
         };
         cudaError_t e = cudaSuccess;
@@ -824,6 +827,7 @@ int nsg_dc_batch_run(nsg_dc_batch* b, const double* d_params, double* d_solution
             b->drop_graph();  // plans and workspace move
             int rc = refresh_plans(b->topos, &b->d_lu_pool, &b->d_plans, &b->max_col, &b->max_n);
             if (rc != NSG_OK) return rc;
+            need = plan_stage(b->topos, false);
             if (nsg::dc_smem_bytes(b->max_col, b->max_n) > 200 * 1024)
                 return fail(NSG_ERR_INVALID, "nsg_dc_batch_run: re-ordered instance too large "
                                              "for the shared-memory refactor");
@@ -836,8 +840,8 @@ int nsg_dc_batch_run(nsg_dc_batch* b, const double* d_params, double* d_solution
                                            static_cast<int>(subset.size()), b->d_prog, params,
                                            b->d_work, d_solutions, d_status, d_iterations,
                                            b->d_ctl, b->opt, b->max_col, b->max_n,
-                                           max_stage_len(b->descs), rmaps, st)) !=
-                    cudaSuccess)
+                                           max_stage_len(b->descs), need.doubles, need.words,
+                                           rmaps, st)) != cudaSuccess)
                 return cuda_fail("nsg_dc_batch_run", e);
         }
         return NSG_OK;

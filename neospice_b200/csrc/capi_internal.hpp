@@ -143,6 +143,13 @@ inline int64_t max_stage_len(const std::vector<nsg::DcDesc>& ds) {
     return m;
 }
 
+// Shared memory the plans of a batch ask of a Newton kernel: the largest
+// level program's working space and the largest staged part of a plan.
+struct PlanStage {
+    int doubles, words;
+};
+PlanStage plan_stage(const std::vector<std::unique_ptr<nsg_topology>>& topos, bool transposed);
+
 // Host (re-)ordering of one instance that stopped on the device.
 // reorder_instance: a copy of topos[topo]'s engine runs NeoSolver::numeric on
 // the instance's matrix values (re-validate, re-order from the failing

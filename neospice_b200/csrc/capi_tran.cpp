@@ -34,7 +34,8 @@ cudaError_t launch_tran_adjoint(const PlanDesc* plans, const int32_t* lu_pool, c
                                 const StepRecord* recs, const double* times, const double* rec_x0,
                                 const double* targets, double weight, double* grads, double* loss,
                                 int32_t* status, const NewtonOptions& opt, int max_iter,
-                                int max_col, int max_n, cudaStream_t stream);
+                                int max_col, int max_n, int lp_doubles, int plan_words,
+                                cudaStream_t stream);
 }  // namespace nsg
 
 using namespace nsg_internal;
@@ -122,12 +123,14 @@ namespace {
 
 // Launch shape of a transient batch (nsg::TranShape).
 nsg::TranShape tran_shape(const nsg_tran_batch& b) {
-    nsg::TranShape sh{b.max_col, b.max_n, max_stage_len(b.descs), 0, 0, 0,
+    nsg::TranShape sh{b.max_col, b.max_n, max_stage_len(b.descs), 0, 0, 0, 0,
                       b.force_threads, b.force_blocks};
-    for (const auto& t : b.topos) {
-        sh.max_small_lu = std::max(sh.max_small_lu, t->plan.nnz_lu + t->plan.n);
-        sh.max_plan_words = std::max<int64_t>(sh.max_plan_words, t->plan.device_words());
-    }
+    const PlanStage need = plan_stage(b.topos, false);
+    sh.lp_doubles = need.doubles;
+    sh.plan_words = need.words;
+    for (const auto& t : b.topos)
+        sh.max_small_lu = std::max({sh.max_small_lu, t->plan.nnz_lu + t->plan.n,
+                                    t->plan.lp_doubles()});
     for (const auto& d : b.descs)
         sh.max_devices = std::max({sh.max_devices, d.n_mos, d.n_diodes, d.n_caps, d.n_srcs});
     return sh;
@@ -630,6 +633,7 @@ int nsg_tran_batch_adjoint(nsg_tran_batch* b, const int* probe, const double* d_
             return cuda_fail("nsg_tran_batch_adjoint", e);
         int64_t nparam = 0;
         for (auto c : b->param_count) nparam += c;
+        const PlanStage need = plan_stage(b->topos, true);
         if ((e = cudaMemcpy(b->d_adescs, ad.data(), sizeof(nsg::AdjDesc) * b->count,
                             cudaMemcpyHostToDevice)) != cudaSuccess ||
             (e = cudaMemsetAsync(d_grads, 0, sizeof(double) * nparam, st)) != cudaSuccess ||
@@ -638,7 +642,8 @@ int nsg_tran_batch_adjoint(nsg_tran_batch* b, const int* probe, const double* d_
                  b->d_prog, d_params_dc ? d_params_dc : b->d_params_dc,
                  d_params_tran ? d_params_tran : b->d_params_tran, b->d_work, b->d_adj_ws,
                  b->d_rec, b->d_times, b->d_x0, d_targets, weight, d_grads, d_loss, d_status,
-                 b->adj_opt, b->adj_max_iter, b->max_col, b->max_n, st)) != cudaSuccess)
+                 b->adj_opt, b->adj_max_iter, b->max_col, b->max_n, need.doubles, need.words,
+                 st)) != cudaSuccess)
             return cuda_fail("nsg_tran_batch_adjoint", e);
         return NSG_OK;
     });

@@ -7,6 +7,7 @@
 #include <atomic>
 #include <cstring>
 #include <functional>
+#include <queue>
 #include <stdexcept>
 #include <string>
 #include <thread>
@@ -35,6 +36,125 @@ void level_sort(const std::vector<int32_t>& level, std::vector<int32_t>& ptr,
     for (int32_t i = 0; i < static_cast<int32_t>(level.size()); ++i)
         members[fill[level[i]]++] = i;
 }
+
+// Bounds of a level program: what it works in and its packed words stay small
+// enough for several CTAs per SM, and its entries' operand chains short (a
+// denser factor has entries with long sums that one lane would walk alone).
+// Inverter chains, BSIM4v7 rings and interconnect trees have 1 to 10 updates
+// per unknown; the 257-unknown mesh has 83 and its columns keep 16 warps busy.
+constexpr int32_t kLevelMaxDoubles = 6144;
+constexpr int64_t kLevelMaxUpdatesPerRow = 32;
+constexpr size_t kLevelMaxWords = 16384;
+constexpr int64_t kPlanStageWords = 4096;  // of a plan without a program
+
+// One section of a level program: entries scheduled into steps of up to 32
+// whose operands were all finished in earlier steps.
+struct LevelBuilder {
+    struct Term {
+        int32_t first, scale, second;
+    };
+    struct Entry {
+        int32_t target, aux, nterms;
+        uint32_t flags;
+        Term terms[kLevelTerms];
+    };
+    std::vector<Entry> entries;
+
+    // The sum over terms[0 .. n - 1] into `target`, as one entry or several:
+    // first_aux goes to the first of them, last_aux and last_flags to the
+    // last, `one` to the others' aux, flags to all.
+    void sum(int32_t target, const Term* terms, int32_t n, int32_t one, int32_t first_aux,
+             int32_t last_aux, uint32_t flags, uint32_t last_flags) {
+        for (int32_t k = 0; k == 0 || k < n; k += kLevelTerms) {
+            const bool last = k + kLevelTerms >= n;
+            Entry e{target, one, std::min(kLevelTerms, n - k), flags, {}};
+            if (k == 0 && first_aux != one) e.aux = first_aux;
+            if (last && last_aux != one) e.aux = last_aux;
+            if (last) e.flags |= last_flags;
+            for (int32_t u = 0; u < e.nterms; ++u) e.terms[u] = terms[k + u];
+            entries.push_back(e);
+        }
+    }
+
+    // Longest remaining chain first (cycles on a B200: about 120 for a step, 110
+    // more for a reciprocal).  values: size of the value space; zero: its
+    // zero.  Appends entry and term words and the steps (offsets relative to
+    // the appended words).
+    void schedule(int32_t values, int32_t zero, std::vector<LevelStep>& steps,
+                  std::vector<uint32_t>& entry_words, std::vector<uint32_t>& term_words) const {
+        const int32_t m = static_cast<int32_t>(entries.size());
+        // the last entry of each value, and of each entry the one before it
+        std::vector<int32_t> maker(values, -1), before(m, -1);
+        for (int32_t e = 0; e < m; ++e) {
+            before[e] = maker[entries[e].target];
+            maker[entries[e].target] = e;
+        }
+        std::vector<int32_t> missing(m, 0), ptr(m + 1, 0);
+        auto operands = [&](int32_t e, auto&& f) {
+            const Entry& x = entries[e];
+            if (before[e] >= 0) f(before[e]);
+            for (int32_t k = 0; k < x.nterms; ++k)
+                for (int32_t v : {x.terms[k].first, x.terms[k].scale, x.terms[k].second})
+                    if (maker[v] >= 0) f(maker[v]);
+        };
+        for (int32_t e = 0; e < m; ++e)
+            operands(e, [&](int32_t o) {
+                ++ptr[o + 1];
+                ++missing[e];
+            });
+        for (int32_t e = 0; e < m; ++e) ptr[e + 1] += ptr[e];
+        std::vector<int32_t> users(ptr[m]), fill(ptr.begin(), ptr.end() - 1);
+        for (int32_t e = 0; e < m; ++e) operands(e, [&](int32_t o) { users[fill[o]++] = e; });
+        std::vector<int32_t> topo, left(missing);
+        topo.reserve(m);
+        for (int32_t e = 0; e < m; ++e)
+            if (left[e] == 0) topo.push_back(e);
+        for (size_t k = 0; k < topo.size(); ++k)
+            for (int32_t u = ptr[topo[k]]; u < ptr[topo[k] + 1]; ++u)
+                if (--left[users[u]] == 0) topo.push_back(users[u]);
+        if (static_cast<int32_t>(topo.size()) != m)
+            throw std::logic_error("plan: level program has a cycle");
+        std::vector<int32_t> height(m, 0);
+        for (int32_t k = m - 1; k >= 0; --k) {
+            const int32_t e = topo[k];
+            int32_t h = 0;
+            for (int32_t u = ptr[e]; u < ptr[e + 1]; ++u) h = std::max(h, height[users[u]]);
+            height[e] = h + 120 + ((entries[e].flags & kLevelPivot) ? 110 : 0);
+        }
+        std::priority_queue<std::pair<int32_t, int32_t>> ready;
+        for (int32_t e = 0; e < m; ++e)
+            if (missing[e] == 0) ready.push({height[e], -e});
+        std::vector<int32_t> step;
+        while (!ready.empty()) {
+            step.clear();
+            while (!ready.empty() && step.size() < 32) {
+                step.push_back(-ready.top().second);
+                ready.pop();
+            }
+            uint32_t pivots = 0;
+            const uint32_t entry_at = static_cast<uint32_t>(4 * entry_words.size());
+            for (int32_t e : step) {
+                pivots |= entries[e].flags & kLevelPivot;
+                entry_words.push_back(static_cast<uint32_t>(8 * entries[e].target) |
+                                      entries[e].flags |
+                                      (static_cast<uint32_t>(8 * entries[e].aux) << 16));
+            }
+            steps.push_back({entry_at, static_cast<uint32_t>(4 * term_words.size()),
+                             static_cast<uint32_t>(step.size()) - 1, pivots});
+            for (int32_t k = 0; k < kLevelTerms; ++k)
+                for (int32_t e : step) {
+                    const Term t = k < entries[e].nterms ? entries[e].terms[k]
+                                                         : Term{zero, zero, zero};
+                    term_words.push_back(static_cast<uint32_t>(8 * t.first) |
+                                         (static_cast<uint32_t>(8 * t.scale) << 16));
+                    term_words.push_back(static_cast<uint32_t>(8 * t.second));
+                }
+            for (int32_t e : step)
+                for (int32_t u = ptr[e]; u < ptr[e + 1]; ++u)
+                    if (--missing[users[u]] == 0) ready.push({height[users[u]], -users[u]});
+        }
+    }
+};
 
 // Derive everything from the CSC LU pattern (col_ptr/row_idx/lu_src set).
 void finish(TopologyPlan& p) {
@@ -232,6 +352,103 @@ void finish(TopologyPlan& p) {
 
 }  // namespace
 
+// The level program of a Markowitz plan (see TopologyPlan::lp), for factors
+// within the bounds above.  An entry of the factor receives its updates in
+// ascending pivot order, a row of a sweep its columns in the order of the
+// row-wise sweeps, so every value is the one the column-wise refactor and the
+// sweeps compute.
+void build_level_program(TopologyPlan& p) {
+    p.lp.clear();
+    p.lp_core = 0;
+    const int32_t n = p.n, nlu = p.nnz_lu;
+    const int32_t vec = nlu, pivots = nlu + n, zero = nlu + 2 * n, one = zero + 1;
+    static_assert(8 * kLevelMaxDoubles <= 0xffff, "value offsets are 16 bits");
+    if (p.kind != kPlanKindMarkowitz || one >= kLevelMaxDoubles ||
+        p.updates > kLevelMaxUpdatesPerRow * n || p.nnz_a >= 0xffff)
+        return;
+    // updates of each LU position, ascending in the source column
+    std::vector<int32_t> upd_ptr(nlu + 1, 0);
+    auto each_update = [&](auto&& f) {
+        for (int32_t j = 0; j < n; ++j)
+            for (int32_t q = p.col_ptr[j]; q < p.diag_pos[j]; ++q) {
+                const int32_t r = p.row_idx[q], cnt = p.col_ptr[r + 1] - p.diag_pos[r] - 1;
+                for (int32_t k = 0; k < cnt; ++k)
+                    f(p.col_ptr[j] + p.upd_dst[p.upd_start[q] + k],
+                      LevelBuilder::Term{q, p.diag_pos[r], p.diag_pos[r] + 1 + k});
+            }
+    };
+    each_update([&](int32_t d, const LevelBuilder::Term&) { ++upd_ptr[d + 1]; });
+    for (int32_t q = 0; q < nlu; ++q) upd_ptr[q + 1] += upd_ptr[q];
+    std::vector<LevelBuilder::Term> upd(upd_ptr[nlu]);
+    std::vector<int32_t> at(upd_ptr.begin(), upd_ptr.end() - 1);
+    each_update([&](int32_t d, const LevelBuilder::Term& t) { upd[at[d]++] = t; });
+    LevelBuilder factor, backward, over_u, over_l;
+    for (int32_t j = 0; j < n; ++j)
+        for (int32_t q = p.col_ptr[j]; q < p.col_ptr[j + 1]; ++q) {
+            const LevelBuilder::Term* t = upd.data() + upd_ptr[q];
+            const int32_t cnt = upd_ptr[q + 1] - upd_ptr[q];
+            if (q == p.diag_pos[j]) factor.sum(q, t, cnt, one, one, pivots + j, 0, kLevelPivot);
+            else if (cnt > 0) factor.sum(q, t, cnt, one, one, one, 0, 0);
+        }
+    std::vector<LevelBuilder::Term> row;
+    for (int32_t i = 0; i < n; ++i) {
+        const int32_t di = p.diag_pos[i];
+        row.clear();
+        for (int32_t k = p.lrow_ptr[i]; k < p.lrow_ptr[i + 1]; ++k)
+            row.push_back({vec + p.lrow_col[k], p.diag_pos[p.lrow_col[k]], p.lrow_pos[k]});
+        if (!row.empty())
+            factor.sum(vec + i, row.data(), static_cast<int32_t>(row.size()), one, one, one,
+                       kLevelSkip, 0);
+        row.clear();
+        for (int32_t k = p.urow_ptr[i]; k < p.urow_ptr[i + 1]; ++k)
+            row.push_back({p.urow_pos[k], di, vec + p.urow_col[k]});
+        backward.sum(vec + i, row.data(), static_cast<int32_t>(row.size()), one, di, one, 0, 0);
+        row.clear();
+        for (int32_t q = p.col_ptr[i]; q < di; ++q)
+            row.push_back({q, p.diag_pos[p.row_idx[q]], vec + p.row_idx[q]});
+        if (!row.empty())
+            over_u.sum(vec + i, row.data(), static_cast<int32_t>(row.size()), one, one, one, 0, 0);
+        row.clear();
+        for (int32_t q = di + 1; q < p.col_ptr[i + 1]; ++q)
+            row.push_back({q, one, vec + p.row_idx[q]});
+        over_l.sum(vec + i, row.data(), static_cast<int32_t>(row.size()), one, one, di, 0, 0);
+    }
+    std::vector<LevelStep> steps;
+    std::vector<uint32_t> ent[4], trm[4];
+    const LevelBuilder* section[4] = {&factor, &backward, &over_u, &over_l};
+    for (int s = 0; s < 4; ++s) {
+        section[s]->schedule(one + 1, zero, steps, ent[s], trm[s]);
+        p.lp_steps[s] = static_cast<int32_t>(steps.size());
+    }
+    std::vector<int32_t>& lp = p.lp;
+    lp.assign(4 * steps.size(), 0);
+    p.lp_src = static_cast<int32_t>(lp.size());
+    p.lp_perm = p.lp_src + (nlu + 1) / 2;
+    lp.resize(p.lp_perm + n, 0);
+    for (int32_t q = 0; q < nlu; ++q) {
+        const uint32_t v = p.lu_src[q] < 0 ? 0xffffu : static_cast<uint32_t>(p.lu_src[q]);
+        lp[p.lp_src + q / 2] |= static_cast<int32_t>(v << (16 * (q % 2)));
+    }
+    for (int32_t i = 0; i < 2 * n; ++i) {
+        const uint32_t v = static_cast<uint32_t>(i < n ? p.perm_row[i] : p.perm_col[i - n]);
+        lp[p.lp_perm + i / 2] |= static_cast<int32_t>(v << (16 * (i % 2)));
+    }
+    for (int s = 0; s < 4; ++s) {
+        if (lp.size() % 2) lp.push_back(0);
+        const uint32_t t0 = static_cast<uint32_t>(4 * lp.size());
+        const uint32_t e0 = t0 + static_cast<uint32_t>(4 * trm[s].size());
+        for (int32_t r = s == 0 ? 0 : p.lp_steps[s - 1]; r < p.lp_steps[s]; ++r) {
+            steps[r].entries += e0;
+            steps[r].terms += t0;
+        }
+        lp.insert(lp.end(), trm[s].begin(), trm[s].end());
+        lp.insert(lp.end(), ent[s].begin(), ent[s].end());
+        if (s == 1) p.lp_core = static_cast<int32_t>(lp.size());
+    }
+    std::memcpy(lp.data(), steps.data(), sizeof(LevelStep) * steps.size());
+    if (lp.size() > kLevelMaxWords) lp.clear();
+}
+
 // Order of the arrays in the device pool; must match PlanArrays in the
 // kernels' header.
 #define NSG_PLAN_ARRAYS(X)                                                      \
@@ -239,7 +456,7 @@ void finish(TopologyPlan& p) {
     X(upd_start) X(upd_dst) X(lrow_ptr) X(lrow_pos) X(lrow_col) X(urow_ptr)     \
     X(urow_pos) X(urow_col) X(col_lev_ptr) X(col_lev) X(fwd_lev_ptr) X(fwd_lev) \
     X(bwd_lev_ptr) X(bwd_lev) X(tbw_lev_ptr) X(tbw_lev) X(rowcopy_pos) X(umeta) \
-    X(piv_rank) X(gmin_pos)
+    X(piv_rank) X(gmin_pos) X(lp)
 
 namespace {
 template <class V>
@@ -262,6 +479,11 @@ void append_packed16(std::vector<int32_t>& pool, const V& v) {
     }
 }
 }  // namespace
+
+int32_t TopologyPlan::stage_words(bool transposed) const {
+    if (!lp.empty()) return transposed ? static_cast<int32_t>(lp.size()) : lp_core;
+    return n <= 128 && device_words() <= kPlanStageWords ? static_cast<int32_t>(device_words()) : 0;
+}
 
 // A packed update map takes one int32 word per two positions.
 int64_t TopologyPlan::device_words() const {

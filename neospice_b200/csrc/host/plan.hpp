@@ -111,6 +111,34 @@ struct TopologyPlan {
     // column's own diagonal element of A), or -1 when the column has none.
     std::vector<int32_t> piv_rank, gmin_pos;
 
+    // Level program (build_level_program; empty when the plan has none): the
+    // refactor and the sweeps of a small sparse factor as steps of up to 32
+    // independent entries, packed into words that a kernel keeps in shared
+    // memory.  It works on unscaled values (a U entry is multiplied by its
+    // pivot's reciprocal where it is used), named by their byte offset in the
+    // kernel's space: the LU positions, the vector (n), the pivots (n), a zero,
+    // a one.  An entry subtracts up to kLevelTerms terms from one value; longer
+    // sums are several entries, one after another.  Layout in words: LevelStep
+    // of every step (four words); lu_src (uint16 per LU position, 0xffff for a
+    // fill-in), perm_row and perm_col (uint16); per section the terms (two
+    // words each: first | scale << 16, second) and entries (one word each:
+    // target | LevelFlag bits, aux << 16) of its steps; lp_core words up to
+    // the transposed sections.  Of a step of w entries, term k of entry e is
+    // at k * w + e, short entries padded with (zero, zero, zero), which
+    // subtracts +0.0.
+    std::vector<int32_t> lp;
+    int32_t lp_core = 0;
+    // Step ends: factor and forward sweep, backward sweep, transposed sweep
+    // over U, over L.
+    int32_t lp_steps[4] = {0, 0, 0, 0};
+    int32_t lp_src = 0, lp_perm = 0;   // word offsets
+    // Doubles of shared memory the program works in.
+    int32_t lp_doubles() const { return lp.empty() ? 0 : nnz_lu + 2 * n + 2; }
+    // Words of the plan that a kernel keeps in shared memory: the level
+    // program (with the transposed section if asked for), else all arrays of a
+    // plan of at most 128 unknowns, else none.
+    int32_t stage_words(bool transposed) const;
+
     // Algorithmic work: multiply-subtract updates of one refactor (each is
     // 2 flops), and the reciprocal pivots.
     int64_t updates = 0;
@@ -133,6 +161,22 @@ struct TopologyPlan {
     void append_to(std::vector<int32_t>& pool, int64_t* off) const;
 };
 
+// One step of a level program: byte offsets of its entries and terms from the
+// program's start, entries - 1, and whether any entry is a pivot.
+struct LevelStep {
+    uint32_t entries, terms, last, pivots;
+};
+constexpr int32_t kLevelTerms = 2;
+
+// An entry computes t = value - sum (first * scale) * second over its terms, in
+// order, and stores t.  The backward sweep starts from value * aux's value
+// unless value is zero; the transposed sweep over L stores t * aux's value
+// (aux is the one where an entry has no such factor).  In the factor section:
+enum LevelFlag : uint32_t {
+    kLevelPivot = 1,  // t itself to aux, 1 / t to the target
+    kLevelSkip = 2,   // forward sweep: terms with first or first * scale zero are left out
+};
+
 // Build from the host ordering engine after order_and_factor.  slot_elem[k]
 // is the engine element of caller CSC slot k.
 TopologyPlan build_plan(const MarkowitzOrder& mo, const std::vector<int32_t>& slot_elem);
@@ -140,6 +184,11 @@ TopologyPlan build_plan(const MarkowitzOrder& mo, const std::vector<int32_t>& sl
 // Build from the AMD-LU engine after a successful factor(): the pivot
 // sequence, L/U structure and replay order of AmdLuSolver::factor_.
 TopologyPlan build_plan_amd(const AmdLuFactor& f);
+
+// Give a plan its level program (TopologyPlan::lp) if it is a small sparse
+// Markowitz plan; clears it otherwise.  The batches of circuits call it for
+// each distinct plan they keep.
+void build_level_program(TopologyPlan& p);
 
 // Build from an exported structure (the reference's own NeoSolver state):
 // elements column by column in internal order (1-based rows/cols), the slot

@@ -11,7 +11,7 @@ enum PlanArray : int {
     PA_upd_start, PA_upd_dst, PA_lrow_ptr, PA_lrow_pos, PA_lrow_col, PA_urow_ptr,
     PA_urow_pos, PA_urow_col, PA_col_lev_ptr, PA_col_lev, PA_fwd_lev_ptr, PA_fwd_lev,
     PA_bwd_lev_ptr, PA_bwd_lev, PA_tbw_lev_ptr, PA_tbw_lev, PA_rowcopy_pos, PA_umeta,
-    PA_piv_rank, PA_gmin_pos, PA_COUNT
+    PA_piv_rank, PA_gmin_pos, PA_lp, PA_COUNT
 };
 
 struct PlanDesc {
@@ -25,6 +25,11 @@ struct PlanDesc {
                            // (every column is shorter than 65,537 rows)
     int64_t off[PA_COUNT];  // int32-word offsets into the plan pool
     int64_t words;          // words from off[0] that hold all of the plan's arrays
+    // Level program (PA_lp; lp_words 0: none): section ends in steps and
+    // word offsets of its parts (TopologyPlan); lp_at: its copy in shared
+    // memory, set by a kernel that made one.
+    int32_t lp_words, lp_core, lp_steps[4], lp_src, lp_perm;
+    const int32_t* lp_at;
 };
 
 #ifdef __CUDACC__

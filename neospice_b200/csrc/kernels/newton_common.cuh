@@ -336,29 +336,30 @@ __device__ inline void assemble(const Inst& v) {
     }
 }
 
-// Shared memory reserved for a staged plan (stage_plan) by the kernels that
-// run many Newton iterations per launch on small instances.
-constexpr size_t kPlanStageBytes = 16 * 1024;
-
-// Copy a plan's index arrays into shared memory (whole CTA) when the
-// instance takes the shared-memory LU path (n <= 128) and the arrays fit
-// cap_words: the refactor and the sweeps read them every Newton iteration,
-// thousands of times per launch in a transient.  Returns the pool to read
-// the plan from; *out (shared) receives the plan descriptor rebased on it.
-// Begins and ends with __syncthreads().
+// Copy what the Newton loop reads of a plan every iteration into shared memory
+// (whole CTA) when it fits cap_words: the level program (with the transposed
+// section if asked for), or all index arrays of a small instance without one.
+// Returns the pool to read the plan's arrays from; *out (shared) receives the
+// plan descriptor, pointing at the copy.  Begins and ends with
+// __syncthreads().
 __device__ inline const int32_t* stage_plan(const PlanDesc& pd, const int32_t* pool, int32_t* sm,
-                                            int64_t cap_words, PlanDesc* out) {
-    const bool fit = sm && pd.n <= 128 && pd.words > 0 && pd.words <= cap_words;
+                                            int64_t cap_words, PlanDesc* out,
+                                            bool transposed = false) {
+    const bool level = pd.lp_words > 0;
+    const int64_t words = level ? (transposed ? pd.lp_words : pd.lp_core) : pd.words;
+    const bool fit = sm && words > 0 && words <= cap_words && (level || pd.n <= 128);
+    const int32_t* from = pool + (level ? pd.off[PA_lp] : pd.off[0]);
     __syncthreads();
     if (threadIdx.x == 0) {
         *out = pd;
-        if (fit)
+        if (fit && level) out->lp_at = sm;
+        else if (fit)
             for (int k = 0; k < PA_COUNT; ++k) out->off[k] -= pd.off[0];
     }
     if (fit)
-        for (int64_t i = threadIdx.x; i < pd.words; i += blockDim.x) sm[i] = pool[pd.off[0] + i];
+        for (int64_t i = threadIdx.x; i < words; i += blockDim.x) sm[i] = from[i];
     __syncthreads();
-    return fit ? sm : pool;
+    return fit && !level ? sm : pool;
 }
 
 struct NewtonOutcome {
@@ -422,8 +423,10 @@ __device__ inline NewtonOutcome newton(const Inst& v, const PlanDesc& pd, const 
     bool force_numeric = false;
     NewtonOutcome out{kDcNoConvergence, max_iter, -1, 0, 1, 0.0};
     double residual = 0.0;
-    // Small instances keep the LU in shared memory (warp-level refactor and
-    // sweeps); larger ones use the dataflow schedule over global memory.
+    // Small sparse factors run their level program and other small ones a
+    // warp-level refactor and sweeps, both in shared memory; larger ones use
+    // the dataflow schedule over global memory.
+    const bool level = level_ready(pd, smem_doubles);
     const bool small = small_fits(pd.n, pd.nnz_lu, smem_doubles);
     double* lu_s = smem;
     double* w_s = smem + pd.nnz_lu;
@@ -457,7 +460,8 @@ __device__ inline NewtonOutcome newton(const Inst& v, const PlanDesc& pd, const 
                           : numeric ? ((solver->factored && !resumed) ? kCheckNumeric : kCheckNone)
                                     : kCheckRefactor;
         const RefactorResult fr =
-            small ? cta_refactor_small(pd, lu_pool, v.a, v.lu, opt.diag_gmin, check, 1e-3, lu_s)
+            level ? cta_level_factor(pd, lu_pool, v.a, v.x, opt.diag_gmin, check, 1e-3)
+            : small ? cta_refactor_small(pd, lu_pool, v.a, v.lu, opt.diag_gmin, check, 1e-3, lu_s)
                   : cta_refactor_flow(pd, lu_pool, v.a, v.lu, opt.diag_gmin, check, 1e-3, smem,
                                       colbuf, v.lrows, v.urows, v.rmaps, v.rmap_stride);
         if (fr.code == kStatusTimeout) {
@@ -484,7 +488,9 @@ __device__ inline NewtonOutcome newton(const Inst& v, const PlanDesc& pd, const 
             __syncthreads();
             continue;
         }
-        if (small) {
+        if (level) {
+            // solved with the factor
+        } else if (small) {
             cta_solve_small(pd, lu_pool, lu_s, v.x, w_s);
         } else if (!cta_solve_flow(pd, lu_pool, v.lu, v.lrows, v.urows, v.x, smem)) {
             out = {kStatusTimeout, iter + 1, -1, 0, 1};

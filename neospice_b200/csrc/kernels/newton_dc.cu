@@ -91,11 +91,15 @@ cudaError_t launch_newton_dc(const PlanDesc* plans, const int32_t* lu_pool, cons
                              const double* params, double* work, double* solutions,
                              int32_t* status, int32_t* iterations, DcCtl* ctls,
                              const NewtonOptions& opt, int max_col, int max_n,
-                             long long max_stage, int32_t* rmaps, cudaStream_t stream) {
+                             long long max_stage, int lp_doubles, int plan_words,
+                             int32_t* rmaps, cudaStream_t stream) {
     if (count <= 0) return cudaSuccess;
     const int colbuf = (max_col + 31) & ~31;
-    const size_t scratch = (dc_smem_bytes(max_col, max_n) + 15) & ~size_t{15};
-    const size_t plan = (max_n <= 128) ? kPlanStageBytes : 0;
+    const size_t level = sizeof(double) * static_cast<size_t>(lp_doubles);
+    const size_t flow = dc_smem_bytes(max_col, max_n);
+    const size_t scratch = ((flow > level ? flow : level) + 15) & ~size_t{15};
+    size_t plan = (sizeof(int32_t) * static_cast<size_t>(plan_words) + 15) & ~size_t{15};
+    if (scratch + plan > kStageCapBytes) plan = 0;  // read from global memory instead
     const size_t stage = stage_bytes_for(scratch + plan, max_stage);
     const size_t smem = scratch + stage + plan;
     if (smem > 200 * 1024) return cudaErrorInvalidValue;

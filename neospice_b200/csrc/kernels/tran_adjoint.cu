@@ -345,13 +345,19 @@ tran_adjoint_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restric
                     const double* __restrict__ rec_x0, const double* __restrict__ targets,
                     double weight, double* __restrict__ grads, double* __restrict__ loss,
                     int32_t* __restrict__ status, NewtonOptions opt, int max_iter, int colbuf,
-                    int scratch_doubles) {
+                    int scratch_doubles, int plan_words) {
     extern __shared__ double smem[];
     const DcDesc d = descs[blockIdx.x];
     const TranDesc td = tdescs[blockIdx.x];
     const AdjDesc ad = adescs[blockIdx.x];
-    const PlanDesc& dpd = plans[d.plan];
-    const PlanDesc& tpd = plans[td.tran_plan];
+    // The plan in use (the DC solver's for the operating point, the transient
+    // solver's for the steps), its level program in shared memory.
+    __shared__ PlanDesc pd;
+    int32_t* plan_sm = plan_words > 0 ? reinterpret_cast<int32_t*>(smem + scratch_doubles) : nullptr;
+    const int32_t* pool = lu_pool;
+    auto use_plan = [&](int32_t plan) {
+        pool = stage_plan(plans[plan], lu_pool, plan_sm, plan_words, &pd, true);
+    };
     Inst v = make_inst(d, prog, params_tran, work);
     const int32_t n = v.n, ns = d.n_states;
     const int64_t K = ad.every;
@@ -399,7 +405,7 @@ tran_adjoint_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restric
             solver.factored = 1;
         }
         __syncthreads();
-        const NewtonOutcome r = newton(v, tpd, lu_pool, &ctx, opt, max_iter, &solver, smem, colbuf,
+        const NewtonOutcome r = newton(v, pd, pool, &ctx, opt, max_iter, &solver, smem, colbuf,
                                        -1, -1, 1, false, scratch_doubles, true);
         if (r.code != kDcConverged) return false;
         vcopy(v.st[3], v.st[2], ns);
@@ -417,9 +423,24 @@ tran_adjoint_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restric
         return 2.0 * weight * (x[ad.probe] - tg[s]);
     };
 
+    // Factor the assembled matrix / solve its transposed system in place.
+    auto factor = [&]() -> RefactorResult {
+        if (level_ready(pd, scratch_doubles))
+            return cta_level_factor(pd, pool, v.a, nullptr, opt.diag_gmin, kCheckNone, 1e-3);
+        return cta_refactor_flow(pd, pool, v.a, v.lu, opt.diag_gmin, kCheckNone, 1e-3, smem,
+                                 colbuf, v.lrows, v.urows);
+    };
+    auto solve_transposed = [&]() {
+        if (level_ready(pd, scratch_doubles))
+            cta_level_solve_transposed(pd, lam);
+        else
+            cta_solve_transposed(pd, pool, v.lu, lam, w);
+    };
+
     // ---- 1. operating point: re-solved with the replayed parameters by
     // Newton from the recorded x_0 (the DC plan's pivots); states seeded
     // from it
+    use_plan(d.plan);
     v.par = params_dc + d.param_off;
     load_constants(v, opt.gmin);
     vcopy(v.x, rec_x0 + td.x0_off, n);
@@ -437,7 +458,7 @@ tran_adjoint_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restric
     }
     __syncthreads();
     {
-        const NewtonOutcome r0 = newton(v, dpd, lu_pool, &ctx, opt, max_iter, &solver, smem,
+        const NewtonOutcome r0 = newton(v, pd, pool, &ctx, opt, max_iter, &solver, smem,
                                         colbuf, -1, -1, 1, false, scratch_doubles, true);
         if (r0.code != kDcConverged) {
             fail_with(kTranDcFailed);
@@ -473,6 +494,7 @@ tran_adjoint_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restric
     __syncthreads();
 
     // ---- 2. forward replay with checkpoints every K steps
+    use_plan(td.tran_plan);
     v.par = params_tran + d.param_off;
     load_constants(v, opt.gmin);
     double* xprev = seg_x;  // x_{s-1} while replaying
@@ -542,9 +564,7 @@ tran_adjoint_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restric
                 __syncthreads();
             }
             assemble(v);
-            const RefactorResult fr = cta_refactor_flow(tpd, lu_pool, v.a, v.lu, opt.diag_gmin,
-                                                        kCheckNone, 1e-3, smem, colbuf,
-                                                        v.lrows, v.urows);
+            const RefactorResult fr = factor();
             if (fr.code != kStatusOk) {
                 fail_with(fr.code);
                 return;
@@ -583,7 +603,7 @@ tran_adjoint_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restric
             if (v.n_mos > 0)
                 mos_charge_rhs(v, mos_base, xs, x1, cf, eta1, eta2, mu, kap1, cap1, w1, p1, lam);
             __syncthreads();
-            cta_solve_transposed(tpd, lu_pool, v.lu, lam, w);
+            solve_transposed();
             // capacitor adjoints and dL/dC
             for (int32_t k = threadIdx.x; k < v.n_caps; k += blockDim.x) {
                 const int32_t* cr = v.caps + 5 * k;
@@ -615,6 +635,7 @@ tran_adjoint_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restric
     }
 
     // ---- 4. the operating point: DC Jacobian, cotangent from steps 1 and 2
+    use_plan(d.plan);
     const double* x0 = ckpt;  // checkpoint 0 holds the re-solved x_0
     v.par = params_dc + d.param_off;
     load_constants(v, opt.gmin);
@@ -632,8 +653,7 @@ tran_adjoint_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restric
     eval_devices(v, ctx, opt, &s_dev_conv);
     __syncthreads();
     assemble(v);
-    const RefactorResult fr = cta_refactor_flow(dpd, lu_pool, v.a, v.lu, opt.diag_gmin, kCheckNone,
-                                                1e-3, smem, colbuf, v.lrows, v.urows);
+    const RefactorResult fr = factor();
     if (fr.code != kStatusOk) {
         fail_with(fr.code);
         return;
@@ -668,7 +688,7 @@ tran_adjoint_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restric
     if (v.n_mos > 0)
         mos_charge_rhs(v, mos_base, x0, x0, cf0, eta1, eta2, mu, kap1, cap1, w1, p1, lam);
     __syncthreads();
-    cta_solve_transposed(dpd, lu_pool, v.lu, lam, w);
+    solve_transposed();
     if (v.n_mos > 0) {
         mos_charge_update(v, mos_base, x0, x0, cf0, lam, eta1, eta2, mu, kap1, cap1, w1, p1,
                           g);
@@ -686,11 +706,17 @@ cudaError_t launch_tran_adjoint(const PlanDesc* plans, const int32_t* lu_pool, c
                                 const StepRecord* recs, const double* times, const double* rec_x0,
                                 const double* targets, double weight, double* grads, double* loss,
                                 int32_t* status, const NewtonOptions& opt, int max_iter,
-                                int max_col, int max_n, cudaStream_t stream) {
+                                int max_col, int max_n, int lp_doubles, int plan_words,
+                                cudaStream_t stream) {
     if (count <= 0) return cudaSuccess;
     const int colbuf = (max_col + 31) & ~31;
     const size_t a = flow_smem_bytes(colbuf, max_n), b = flow_solve_smem_bytes(max_n);
-    const size_t smem = ((a > b ? a : b) + 15) & ~size_t{15};
+    const size_t level = sizeof(double) * static_cast<size_t>(lp_doubles);
+    const size_t flow = a > b ? a : b;
+    const size_t scratch = ((flow > level ? flow : level) + 15) & ~size_t{15};
+    size_t plan = (sizeof(int32_t) * static_cast<size_t>(plan_words) + 15) & ~size_t{15};
+    if (scratch + plan > kStageCapBytes) plan = 0;  // read from global memory instead
+    const size_t smem = scratch + plan;
     if (smem > 200 * 1024) return cudaErrorInvalidValue;
     static bool configured = false;
     if (!configured) {
@@ -703,7 +729,7 @@ cudaError_t launch_tran_adjoint(const PlanDesc* plans, const int32_t* lu_pool, c
     tran_adjoint_kernel<<<count, kFlowThreads, smem, stream>>>(
         plans, lu_pool, descs, tdescs, adescs, prog, params_dc, params_tran, work, adj_ws, recs,
         times, rec_x0, targets, weight, grads, loss, status, opt, max_iter, colbuf,
-        static_cast<int>(smem / sizeof(double)));
+        static_cast<int>(scratch / sizeof(double)), static_cast<int>(plan / sizeof(int32_t)));
     return cudaGetLastError();
 }
 

@@ -60,13 +60,15 @@ struct TranCtl {
 
 // What the launch needs to size one CTA: the batch's largest LU column and
 // unknown count (dataflow scratch), largest staged workspace, largest
-// small-path LU (nnz_lu + n doubles), largest plan (int32 words) and most
-// devices of one family in one instance (the device loads' parallelism).
+// shared-memory LU (doubles: nnz_lu + n, or a level program's space), largest
+// space of a level program, most words of a plan to keep in shared memory and
+// most devices of one family in one instance (the device loads' parallelism).
 struct TranShape {
     int32_t max_col, max_n;
     int64_t max_stage;
     int32_t max_small_lu;
-    int64_t max_plan_words;
+    int32_t lp_doubles;
+    int32_t plan_words;
     int32_t max_devices;
     int32_t force_threads;   // nsg_tran_batch_set_shape (0: automatic)
     int32_t force_blocks;

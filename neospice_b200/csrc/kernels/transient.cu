@@ -573,17 +573,18 @@ cudaError_t launch_transient(const PlanDesc* plans, const int32_t* lu_pool, cons
     if (small_shape && sh.max_n > 128) return cudaErrorInvalidValue;
     size_t scratch, plan, stage;
     if (!small_shape) {
-        scratch = (tran_smem_bytes(sh.max_col, sh.max_n) + 15) & ~size_t{15};
-        plan = (sh.max_n <= 128) ? kPlanStageBytes : 0;
+        const size_t flow = tran_smem_bytes(sh.max_col, sh.max_n);
+        const size_t level = sizeof(double) * static_cast<size_t>(sh.lp_doubles);
+        scratch = ((flow > level ? flow : level) + 15) & ~size_t{15};
+        plan = (sizeof(int32_t) * static_cast<size_t>(sh.plan_words) + 15) & ~size_t{15};
+        if (scratch + plan > kStageCapBytes) plan = 0;  // read from global memory instead
         stage = stage_bytes_for(scratch + plan, sh.max_stage);
     } else {
         // Per-CTA share of the SM's 228 KB, less the CTA's static shared
         // memory and the 1 KB the runtime reserves per CTA.
         const size_t budget = (228 * 1024) / static_cast<size_t>(blocks) - 3 * 1024;
         scratch = (sizeof(double) * static_cast<size_t>(sh.max_small_lu) + 15) & ~size_t{15};
-        plan = (sh.max_plan_words * 4 <= static_cast<int64_t>(kPlanStageBytes))
-                   ? ((static_cast<size_t>(sh.max_plan_words) * 4 + 15) & ~size_t{15})
-                   : 0;
+        plan = (sizeof(int32_t) * static_cast<size_t>(sh.plan_words) + 15) & ~size_t{15};
         if (scratch + plan > budget) plan = 0;
         const size_t want = static_cast<size_t>(sh.max_stage) * sizeof(double);
         stage = (scratch + plan + want <= budget) ? want : 0;

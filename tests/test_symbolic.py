@@ -92,3 +92,26 @@ def test_order_matches_reference_stress():
         assert _same(topo, st2), f"case {t} renumeric"
         checked += 1
     assert checked > 300
+
+
+def test_level_program_matches_columnwise_refactor(tmp_path):
+    """The level programs of small sparse factors, run step after step on
+    the CPU, give the column-wise refactor, the sweeps and the transposed
+    sweeps bit for bit, with every index in range and no hazard inside a step
+    (tests/cpp/level_program_check.cpp, compiled here from the host sources)."""
+    import pathlib
+    import shutil
+    import subprocess
+    cxx = shutil.which("g++") or shutil.which("c++")
+    if not cxx:
+        pytest.skip("no host C++ compiler")
+    root = pathlib.Path(__file__).resolve().parents[1]
+    src = root / "neospice_b200" / "csrc"
+    exe = tmp_path / "level_program_check"
+    subprocess.run([cxx, "-std=c++17", "-O2", "-ffp-contract=off", "-pthread", f"-I{src}",
+                    str(root / "tests" / "cpp" / "level_program_check.cpp"),
+                    str(src / "host" / "amd_lu.cpp"), str(src / "host" / "plan.cpp"),
+                    str(src / "host" / "sparse_order.cpp"), "-o", str(exe)], check=True)
+    res = subprocess.run([str(exe)], capture_output=True, text=True, timeout=600)
+    assert res.returncode == 0, res.stdout + res.stderr
+    assert "0 failure(s)" in res.stdout
