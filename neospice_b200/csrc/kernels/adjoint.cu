@@ -50,8 +50,10 @@ dc_adjoint_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restrict_
     }
     double* lam = v.x;
     for (int32_t i = threadIdx.x; i < v.n; i += blockDim.x) lam[i] = cotangent[d.sol_off + i];
-    double* w = work + d.w_off;
-    cta_solve_transposed(pd, lu_pool, v.lu, lam, w);
+    if (!cta_solve_transposed_flow(pd, lu_pool, v.lu, lam, smem)) {
+        if (threadIdx.x == 0) status[d.index] = kStatusTimeout;
+        return;
+    }
 
     const int32_t* gp = prog + d.prog_off[DP_grad];
     double* g = grads + d.param_off;
@@ -89,7 +91,8 @@ cudaError_t launch_dc_adjoint(const PlanDesc* plans, const int32_t* lu_pool, con
                               cudaStream_t stream) {
     if (count <= 0) return cudaSuccess;
     const int colbuf = (max_col + 31) & ~31;
-    const size_t smem = flow_smem_bytes(colbuf, max_n);
+    const size_t flow = flow_smem_bytes(colbuf, max_n), sweep = flow_solve_smem_bytes(max_n);
+    const size_t smem = flow > sweep ? flow : sweep;
     if (smem > 200 * 1024) return cudaErrorInvalidValue;
     static bool configured = false;
     if (!configured) {

