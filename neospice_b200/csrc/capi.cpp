@@ -262,6 +262,13 @@ int32_t grid_tail_from(const nsg::TopologyPlan& p) {
     return (p.n - j >= 2) ? j : p.n;
 }
 
+std::vector<int64_t> stage_lens(const std::vector<nsg::DcDesc>& ds) {
+    std::vector<int64_t> lens;
+    for (const auto& d : ds) lens.push_back(d.stage_len);
+    std::sort(lens.begin(), lens.end());
+    return lens;
+}
+
 PlanStage plan_stage(const std::vector<std::unique_ptr<nsg_topology>>& topos, bool transposed) {
     PlanStage s{0, 0};
     for (const auto& t : topos) {

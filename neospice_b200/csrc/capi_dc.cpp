@@ -19,8 +19,8 @@ cudaError_t launch_newton_dc(const PlanDesc* plans, const int32_t* lu_pool, cons
                              const double* params, double* work, double* solutions,
                              int32_t* status, int32_t* iterations, DcCtl* ctls,
                              const NewtonOptions& opt, int max_col, int max_n,
-                             long long max_stage, int lp_doubles, int plan_words,
-                             int32_t* rmaps, cudaStream_t stream);
+                             const int64_t* stage_lens, int n_stage, int lp_doubles,
+                             int plan_words, int32_t* rmaps, cudaStream_t stream);
 size_t dc_smem_bytes(int max_col, int max_n);
 cudaError_t launch_dc_adjoint(const PlanDesc* plans, const int32_t* lu_pool, const DcDesc* descs,
                               int count, const int32_t* prog, const double* params, double* work,
@@ -735,8 +735,7 @@ int nsg_dc_batch_run(nsg_dc_batch* b, const double* d_params, double* d_solution
         const cudaStream_t st = static_cast<cudaStream_t>(stream);
         const double* params = d_params ? d_params : b->d_params;
         if (b->row_maps) {
-            // warps per CTA of newton_dc_kernel (16), max_n words each
-            const int64_t words = int64_t{b->count} * 16 * b->max_n;
+            const int64_t words = int64_t{b->count} * nsg::kDcMaxWarps * b->max_n;
             if (words > b->rmap_cap) {
                 b->drop_graph();
                 cudaFree(b->d_rmap);
@@ -750,13 +749,14 @@ int nsg_dc_batch_run(nsg_dc_batch* b, const double* d_params, double* d_solution
         }
         int32_t* rmaps = b->row_maps ? b->d_rmap : nullptr;
         PlanStage need = plan_stage(b->topos, false);
+        const std::vector<int64_t> lens = stage_lens(b->descs);
         auto first_launch = [&](cudaStream_t s) -> cudaError_t {
             cudaError_t r = cudaMemsetAsync(b->d_ctl, 0, sizeof(nsg::DcCtl) * b->count, s);
             if (r == cudaSuccess)
                 r = nsg::launch_newton_dc(b->d_plans, b->d_lu_pool, b->d_descs, nullptr, b->count,
                                           b->d_prog, params, b->d_work, d_solutions, d_status,
                                           d_iterations, b->d_ctl, b->opt, b->max_col, b->max_n,
-                                          max_stage_len(b->descs), need.doubles, need.words, rmaps, s);
+                                          lens.data(), b->count, need.doubles, need.words, rmaps, s);
             return r;
         };
         cudaError_t e = cudaSuccess;
@@ -840,7 +840,7 @@ int nsg_dc_batch_run(nsg_dc_batch* b, const double* d_params, double* d_solution
                                            static_cast<int>(subset.size()), b->d_prog, params,
                                            b->d_work, d_solutions, d_status, d_iterations,
                                            b->d_ctl, b->opt, b->max_col, b->max_n,
-                                           max_stage_len(b->descs), need.doubles, need.words,
+                                           lens.data(), b->count, need.doubles, need.words,
                                            rmaps, st)) != cudaSuccess)
                 return cuda_fail("nsg_dc_batch_run", e);
         }

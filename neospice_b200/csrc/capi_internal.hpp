@@ -136,12 +136,8 @@ void fill_instance(nsg::DcDesc& d, const nsg::Circuit& c, const nsg::TopologyPla
                    std::vector<int32_t>& prog, int64_t& work);
 // The gmin-stepping save area, placed after the staged regions.
 void place_dcsave(nsg::DcDesc& d, int64_t& work);
-// Largest stage_len over instances (doubles).
-inline int64_t max_stage_len(const std::vector<nsg::DcDesc>& ds) {
-    int64_t m = 0;
-    for (const auto& d : ds) m = d.stage_len > m ? d.stage_len : m;
-    return m;
-}
+// The instances' stage_len (doubles), ascending.
+std::vector<int64_t> stage_lens(const std::vector<nsg::DcDesc>& ds);
 
 // Shared memory the plans of a batch ask of a Newton kernel: the largest
 // level program's working space and the largest staged part of a plan.

@@ -123,8 +123,8 @@ namespace {
 
 // Launch shape of a transient batch (nsg::TranShape).
 nsg::TranShape tran_shape(const nsg_tran_batch& b) {
-    nsg::TranShape sh{b.max_col, b.max_n, max_stage_len(b.descs), 0, 0, 0, 0,
-                      b.force_threads, b.force_blocks};
+    nsg::TranShape sh{b.max_col, b.max_n, stage_lens(b.descs), 0, 0, 0, 0, b.force_threads,
+                      b.force_blocks};
     const PlanStage need = plan_stage(b.topos, false);
     sh.lp_doubles = need.doubles;
     sh.plan_words = need.words;

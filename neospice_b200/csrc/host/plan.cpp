@@ -296,6 +296,18 @@ void finish(TopologyPlan& p) {
             }
         }
 
+    // next[r]: the column r' whose L rows follow it in L(:, r), if L(:, r) is r'
+    // and then L(:, r') -- neighbours in a run of equal structure.
+    std::vector<int32_t> next(n, -1);
+    for (int32_t r = 0; r < n; ++r) {
+        const int32_t l0 = p.diag_pos[r] + 1, cnt = p.col_ptr[r + 1] - l0;
+        if (cnt == 0) continue;
+        const int32_t r2 = p.row_idx[l0], m0 = p.diag_pos[r2] + 1;
+        if (p.col_ptr[r2 + 1] - m0 == cnt - 1 &&
+            std::equal(p.row_idx.begin() + m0, p.row_idx.begin() + m0 + cnt - 1,
+                       p.row_idx.begin() + l0 + 1))
+            next[r] = r2;
+    }
     p.umeta.assign(4 * static_cast<size_t>(p.nnz_lu), 0);
     for (int32_t j = 0; j < n; ++j)
         for (int32_t q = p.col_ptr[j]; q < p.diag_pos[j]; ++q) {
@@ -303,6 +315,7 @@ void finish(TopologyPlan& p) {
             p.umeta[4 * q] = r;
             p.umeta[4 * q + 1] = p.diag_pos[r];
             p.umeta[4 * q + 2] = p.col_ptr[r + 1] - p.diag_pos[r] - 1;
+            if (q + 1 < p.diag_pos[j] && next[r] == p.row_idx[q + 1]) p.umeta[4 * q + 2] |= kRunBit;
             p.umeta[4 * q + 3] = p.upd_start[q];
         }
     p.rowcopy_pos.assign(p.nnz_lu, -1);

@@ -40,6 +40,8 @@ struct UninitAllocator : std::allocator<T> {
 class MarkowitzOrder;
 class AmdLuFactor;
 
+constexpr int32_t kRunBit = INT32_MIN;  // of TopologyPlan::umeta's third words
+
 // Engines whose pivot sequence a plan replays.
 enum PlanKindHost : int32_t {
     kPlanKindMarkowitz = 0,  // SparseMatrix (Sparse 1.3): U scaled by 1/pivot
@@ -90,7 +92,9 @@ struct TopologyPlan {
     std::vector<int32_t> rowcopy_pos;
     // Per LU position q of a U entry (r, j): {r, diag_pos[r], |L(:, r)|,
     // upd_start[q]} packed as four int32 (zeros elsewhere), so one 16-byte
-    // load gives the refactor everything it needs to apply entry q.
+    // load gives the refactor everything it needs to apply entry q.  The third
+    // has its top bit (kRunBit) set when entry q + 1 = (r', j) continues a
+    // run: L(:, r) is r' followed by L(:, r') in stored order.
     std::vector<int32_t> umeta;
 
     // Level schedules (ptr over levels, then members sorted by level).

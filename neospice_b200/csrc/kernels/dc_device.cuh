@@ -58,6 +58,9 @@ struct NewtonOptions {
 
 enum : int32_t { kAidDirect = 0, kAidSource = 1, kAidGain = 2, kAidPseudoTransient = 3 };
 
+// Most warps of a newton_dc_kernel CTA (the row maps are sized for them).
+constexpr int kDcMaxWarps = 24;
+
 constexpr int kDiodeTermCount = 5;
 constexpr int kCapTermCount = 4;
 constexpr int kSrcTermCount = 2;

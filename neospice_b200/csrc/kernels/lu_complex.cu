@@ -86,7 +86,7 @@ complex_refactor_kernel(const PlanDesc* __restrict__ plans, const int32_t* __res
         __syncwarp();
         bool timed_out = false;
         for (int32_t q = 0; q < dj; ++q) {
-            const int4 m = umeta[c0 + q];  // {r, diag_pos[r], |L(:, r)|, upd_start}
+            const int4 m = u_entry(umeta, c0 + q);  // {r, diag_pos[r], |L(:, r)|, upd_start}
             int ready = 0;
             if (lane == 0) {
                 int spins = 0;

@@ -39,7 +39,14 @@ cudaError_t set_wait_limit_here(int polls) {
 const bool wait_limit_setter_registered = register_wait_limit_setter(&set_wait_limit_here);
 }  // namespace
 // Rounds of 32 L(:, r) rows the dataflow refactor loads before applying them.
-constexpr int kColChunk = 4;
+constexpr int kColChunk = 2;
+// Entries whose completion flags a refactoring warp looks at together, entries
+// of a run it applies together, and other entries whose operands it loads
+// together.  More of each (8, 8, 4) costs registers: at 64 a thread the
+// spills took back more than the longer runs gave.
+constexpr int kRunLanes = 4;
+constexpr int kRun = 4;
+constexpr int kGroup = 2;
 
 __device__ __forceinline__ double lu_mul(double x, double y) { return __dmul_rn(x, y); }
 __device__ __forceinline__ double lu_sub(double x, double y) { return __dsub_rn(x, y); }
@@ -189,10 +196,10 @@ __device__ __forceinline__ unsigned long long fail_key(int32_t step, int32_t cod
            static_cast<uint32_t>(code);
 }
 
-// Shared memory of the dataflow refactor: kFlowWarps column buffers of
-// colbuf doubles, then n int32 completion flags.
-__host__ __device__ inline size_t flow_smem_bytes(int colbuf, int n) {
-    return sizeof(double) * kFlowWarps * colbuf + sizeof(int32_t) * n;
+// Shared memory of the dataflow refactor: a column buffer of colbuf doubles per
+// warp, then n int32 completion flags.
+__host__ __device__ inline size_t flow_smem_bytes(int colbuf, int n, int warps = kFlowWarps) {
+    return sizeof(double) * warps * colbuf + sizeof(int32_t) * n;
 }
 
 struct RefactorResult {
@@ -216,6 +223,64 @@ __device__ __forceinline__ double lu_peer(const double* p) {
     return *p;
 }
 
+// Where a column's update destinations come from: the packed update map, or
+// per-warp row maps.
+enum DestKind : int { kDestMap16 = 0, kDestRowMap = 1 };
+
+// kRun consecutive U entries (r_0, j), (r_1, j), ... of column j that form a
+// run -- L(:, r_i) is r_(i+1) and then L(:, r_(i+1)) -- at positions q .. q +
+// kRun - 1 of the column in buf, applied together by one warp.  Entry i's
+// updates of the other entries of the run are a small triangle, done in
+// registers (lane i holds entry i); below it all kRun columns have the same
+// rows, so a row's value is read and written once, receives its kRun updates in
+// ascending order, and its kRun factors are independent loads in flight
+// together.  Of a mesh's updates nine in ten lie in such runs.  dp:
+// diag_pos[r_(lane % kRun)]; cnt, us: |L(:, r)| and upd_start of the last
+// entry.  Ends with __syncwarp().
+template <bool kCrossSm, class Dest>
+__device__ __forceinline__ void run_step(bool amd, const double* lu, double* buf, int32_t q,
+                                         int32_t dp, int32_t cnt, int32_t us, Dest dest,
+                                         double& colmax) {
+    const int lane = threadIdx.x & 31;
+    int32_t at[kRun];  // diag_pos of each entry's column
+#pragma unroll
+    for (int i = 0; i < kRun; ++i) at[i] = __shfl_sync(0xffffffffu, dp, i);
+    const int32_t l0 = at[kRun - 1] + 1;
+    double x = lane < kRun ? buf[q + lane] : 0.0;
+    const double rd = (lane < kRun && !amd) ? lu_peer<kCrossSm>(lu + dp) : 0.0;
+    double tri[kRun], l[kRun], u[kRun];
+    int32_t d;
+#pragma unroll
+    for (int i = 0; i < kRun - 1; ++i)
+        tri[i] = (lane > i && lane < kRun) ? lu_peer<kCrossSm>(lu + at[i] + lane - i) : 0.0;
+    auto load = [&](int32_t t) {
+        d = t < cnt ? dest(us, l0, t) : 0;
+#pragma unroll
+        for (int i = 0; i < kRun; ++i)
+            l[i] = t < cnt ? lu_peer<kCrossSm>(lu + at[i] + (kRun - i) + t) : 0.0;
+    };
+    load(lane);
+#pragma unroll
+    for (int i = 0; i < kRun; ++i) {
+        const double v = amd ? x : lu_mul(x, rd);
+        u[i] = __shfl_sync(0xffffffffu, v, i);
+        if (lane == i) x = v;
+        if (i < kRun - 1 && lane > i) x = lu_sub(x, lu_mul(u[i], tri[i]));
+        colmax = fmax(colmax, fabs(u[i]));
+    }
+    if (lane < kRun) buf[q + lane] = x;
+    for (int32_t t = lane; t < cnt + lane; t += 32) {
+        if (t >= 32) load(t);
+        if (t < cnt) {
+            double v = buf[d];
+#pragma unroll
+            for (int i = 0; i < kRun; ++i) v = lu_sub(v, lu_mul(u[i], l[i]));
+            buf[d] = v;
+        }
+    }
+    __syncwarp();
+}
+
 // Column j of the left-looking dataflow refactor, by one warp.  buf holds the
 // column while it is eliminated (shared memory, or the column's own place in
 // lu); probe(r) reads column r's completion flag (acquire).  Loads A
@@ -228,18 +293,18 @@ __device__ __forceinline__ double lu_peer(const double* p) {
 // warp's row -> position scratch (pd.n words), written for column j's rows
 // first.  The row map reads L(:, r)'s row indices, which every consumer
 // column of r shares, instead of a map entry per update.
-template <bool kCrossSm, class Probe, int kChunk = kColChunk>
-__device__ __forceinline__ ColumnResult refactor_column(
+template <bool kCrossSm, int kPlan, int kDest, int kChunk = kColChunk, class Probe, class Publish>
+__device__ __forceinline__ void refactor_column(
     const PlanDesc& pd, const int32_t* __restrict__ pool, const double* __restrict__ a,
     double* lu, double diag_gmin, int check_pivots, double rel_threshold, int32_t j, double* buf,
-    double* __restrict__ lrows, double* __restrict__ urows, Probe probe,
+    double* __restrict__ lrows, double* __restrict__ urows, Probe probe, Publish publish,
     int32_t* rmap = nullptr) {
     const int32_t* col_ptr = pool + pd.off[PA_col_ptr];
     const int32_t* diag_pos = pool + pd.off[PA_diag_pos];
     const int32_t* lu_src = pool + pd.off[PA_lu_src];
     const int32_t* upd_dst = pool + pd.off[PA_upd_dst];
-    const int32_t map16 = pd.map16;
-    const bool amd = pd.kind == kPlanAmdLu;
+    const int32_t map16 = kDest == kDestMap16 ? 1 : pd.map16;
+    const bool amd = kPlan < 0 ? pd.kind == kPlanAmdLu : kPlan == kPlanAmdLu;
     const int32_t* piv_rank = pool + pd.off[PA_piv_rank];
     const int32_t* gmin_pos = pool + pd.off[PA_gmin_pos];
     const int lane = threadIdx.x & 31;
@@ -249,7 +314,7 @@ __device__ __forceinline__ ColumnResult refactor_column(
     const int32_t dj = diag_pos[j] - c0;
     const int32_t gp = amd ? gmin_pos[j] : dj;
     const int32_t* row_idx = pool + pd.off[PA_row_idx];
-    const bool mapped = rmap == nullptr;
+    const bool mapped = kDest < 0 ? rmap == nullptr : kDest == kDestMap16;
     for (int32_t t = lane; t < len; t += 32) {
         const int32_t s = lu_src[c0 + t];
         double v = (s >= 0) ? a[s] : 0.0;
@@ -264,103 +329,101 @@ __device__ __forceinline__ ColumnResult refactor_column(
     };
     double colmax = 0.0;  // AMD-LU: largest |U(r, j)| applied
     // U-entry metadata {r, diag_pos[r], |L(:,r)|, upd_start} is held 32
-    // entries at a time in registers (lane k holds entry base+k) and
-    // broadcast by shuffle.  One-step lookahead: while the update of entry q
-    // runs, the pivot reciprocal, the first 32 entries of L(:, r) and their
-    // destinations for entry q+1 are loaded (when column r is done), so a
-    // step waits on at most one global round trip.
+    // entries at a time in registers (lane k holds entry base + k) and
+    // broadcast by shuffle; chain: bit k says that entry base + k + 1 continues
+    // entry base + k's run.
     const int4* umeta = reinterpret_cast<const int4*>(pool + pd.off[PA_umeta]) + c0;
     bool timed_out = false;
-    int4 chunk = make_int4(0, 0, 0, 0), next_chunk = make_int4(0, 0, 0, 0);
-    if (lane < dj) chunk = umeta[lane];
-    if (32 + lane < dj) next_chunk = umeta[32 + lane];
-    double rd_c = 0.0, lv_c = 0.0;
-    int32_t l0_c = 0, cnt_c = 0, us_c = 0, ld_c = 0;
-    bool have_c = false;
-    // Load the operands of entry q (metadata m) if column m.x is done, or
-    // after waiting for it.
-    auto fetch = [&](const int4 m, bool wait, double& rd, double& lv, int32_t& l0, int32_t& cnt,
-                     int32_t& us, int32_t& ld) -> bool {
-        int ready = 0;
-        if (lane == 0) {
-            const int limit = c_wait_limit;
-            int spins = 0;
-            while ((ready = probe(m.x)) == 0 && wait) {
-                if (++spins > limit) {
-                    timed_out = true;
-                    break;
+    int32_t base = 0;
+    int4 meta;
+    unsigned chain;
+    auto window = [&](int32_t at) {
+        base = at;
+        meta = at + lane < dj ? umeta[at + lane] : make_int4(0, 0, 0, 0);
+        chain = __ballot_sync(0xffffffffu, meta.z < 0);
+    };
+    window(0);
+    for (int32_t q = 0; q < dj;) {
+        if (q - base > 32 - kRunLanes && base + 32 < dj) window(q);
+        const int32_t k0 = q - base;
+        // How many of the next entries' source columns are done, at least one.
+        const int32_t ahead = min(min(kRunLanes, dj - q), 32 - k0);
+        const int32_t src = __shfl_sync(0xffffffffu, meta.x, k0 + (lane & (kRunLanes - 1)));
+        int32_t ready = 0;
+        for (int spins = 0;;) {
+            const bool open = lane < ahead && probe(src) == 0;
+            const unsigned mask = __ballot_sync(0xffffffffu, open);
+            ready = mask ? __ffs(mask) - 1 : ahead;
+            if (ready > 0) break;
+            if (++spins > c_wait_limit) {
+                timed_out = true;
+                break;
+            }
+            __nanosleep(64);
+        }
+        if (timed_out) break;
+        __syncwarp();
+        // entries of q's run in the window
+        const int32_t run = __ffs(~(chain >> k0));
+        const int32_t both = min(run, ready);
+        if (both >= kRun) {
+            const int32_t last = k0 + kRun - 1;
+            run_step<kCrossSm>(amd, lu, buf, q,
+                               __shfl_sync(0xffffffffu, meta.y, k0 + (lane & (kRun - 1))),
+                               __shfl_sync(0xffffffffu, meta.z, last) & 0x7fffffff,
+                               __shfl_sync(0xffffffffu, meta.w, last), dest, colmax);
+            q += kRun;
+        } else {
+            // Up to kGroup entries of any structure: the first 32 rows of
+            // every L(:, r), their destinations and the pivot reciprocals
+            // are loaded together, then applied one entry after another.
+            const int32_t count = min(kGroup, ready);
+            int32_t l0[kGroup], cnt[kGroup], us[kGroup], dd[kGroup];
+            double rd[kGroup], ll[kGroup];
+#pragma unroll
+            for (int g = 0; g < kGroup; ++g) {
+                const int32_t k = k0 + min(g, count - 1);
+                const int32_t dp = __shfl_sync(0xffffffffu, meta.y, k);
+                l0[g] = dp + 1;
+                cnt[g] = __shfl_sync(0xffffffffu, meta.z, k) & 0x7fffffff;
+                if (g >= count) cnt[g] = 0;
+                us[g] = __shfl_sync(0xffffffffu, meta.w, k);
+                rd[g] = (amd || g >= count) ? 0.0 : lu_peer<kCrossSm>(lu + dp);
+                ll[g] = lane < cnt[g] ? lu_peer<kCrossSm>(lu + l0[g] + lane) : 0.0;
+                dd[g] = lane < cnt[g] ? dest(us[g], l0[g], lane) : 0;
+            }
+#pragma unroll
+            for (int g = 0; g < kGroup; ++g) {
+                if (g < count) {
+                    const double u = amd ? buf[q + g] : lu_mul(buf[q + g], rd[g]);
+                    colmax = fmax(colmax, fabs(u));
+                    __syncwarp();
+                    if (lane == 0) buf[q + g] = u;
+                    if (lane < cnt[g]) buf[dd[g]] = lu_sub(buf[dd[g]], lu_mul(u, ll[g]));
+                    // rows beyond the first 32, kChunk rounds at a time (the
+                    // destinations of one entry are distinct, so the order
+                    // among them does not matter)
+                    for (int32_t t0 = 32; t0 < cnt[g]; t0 += 32 * kChunk) {
+                        int32_t d[kChunk];
+                        double l[kChunk];
+#pragma unroll
+                        for (int k = 0; k < kChunk; ++k) {
+                            const int32_t t = t0 + 32 * k + lane;
+                            d[k] = (t < cnt[g]) ? dest(us[g], l0[g], t) : 0;
+                            l[k] = (t < cnt[g]) ? lu_peer<kCrossSm>(lu + l0[g] + t) : 0.0;
+                        }
+#pragma unroll
+                        for (int k = 0; k < kChunk; ++k)
+                            if (t0 + 32 * k + lane < cnt[g])
+                                buf[d[k]] = lu_sub(buf[d[k]], lu_mul(u, l[k]));
+                    }
+                    __syncwarp();
                 }
-                __nanosleep(64);
             }
+            q += count;
         }
-        ready = __shfl_sync(0xffffffffu, ready, 0);
-        timed_out = __shfl_sync(0xffffffffu, timed_out, 0);
-        __syncwarp();
-        if (!ready) return false;
-        rd = lu_peer<kCrossSm>(lu + m.y);
-        l0 = m.y + 1;
-        cnt = m.z;
-        us = m.w;
-        lv = (lane < cnt) ? lu_peer<kCrossSm>(lu + l0 + lane) : 0.0;
-        ld = (lane < cnt) ? dest(us, l0, lane) : 0;
-        return true;
-    };
-    auto meta = [&](int32_t q) -> int4 {
-        const int k = q & 31;
-        const int4 src = ((q >> 5) == 0) ? chunk : next_chunk;
-        int4 m;
-        m.x = __shfl_sync(0xffffffffu, src.x, k);
-        m.y = __shfl_sync(0xffffffffu, src.y, k);
-        m.z = __shfl_sync(0xffffffffu, src.z, k);
-        m.w = __shfl_sync(0xffffffffu, src.w, k);
-        return m;
-    };
-    int32_t base = 0;  // entry index held in chunk's lane 0
-    for (int32_t q = 0; q < dj; ++q) {
-        if (q - base == 32) {  // advance the register window by 32 entries
-            base += 32;
-            chunk = next_chunk;
-            next_chunk = (base + 32 + lane < dj) ? umeta[base + 32 + lane] : make_int4(0, 0, 0, 0);
-        }
-        if (!have_c) {
-            fetch(meta(q - base), true, rd_c, lv_c, l0_c, cnt_c, us_c, ld_c);
-            if (timed_out) break;
-        }
-        double rd_n = 0.0, lv_n = 0.0;
-        int32_t l0_n = 0, cnt_n = 0, us_n = 0, ld_n = 0;
-        const bool have_n = (q + 1 < dj) &&
-                            fetch(meta(q + 1 - base), false, rd_n, lv_n, l0_n, cnt_n, us_n, ld_n);
-        const double u = amd ? buf[q] : lu_mul(buf[q], rd_c);
-        colmax = fmax(colmax, fabs(u));
-        __syncwarp();
-        if (lane == 0) buf[q] = u;
-        if (lane < cnt_c) buf[ld_c] = lu_sub(buf[ld_c], lu_mul(u, lv_c));
-        // L(:, r) beyond its first 32 rows: destinations and values are
-        // loaded kChunk rounds at a time before they are applied (the
-        // destinations of one entry are distinct, so the order among them
-        // does not matter).
-        for (int32_t t0 = 32; t0 < cnt_c; t0 += 32 * kChunk) {
-            int32_t dd[kChunk];
-            double ll[kChunk];
-#pragma unroll
-            for (int k = 0; k < kChunk; ++k) {
-                const int32_t t = t0 + 32 * k + lane;
-                dd[k] = (t < cnt_c) ? dest(us_c, l0_c, t) : 0;
-                ll[k] = (t < cnt_c) ? lu_peer<kCrossSm>(lu + l0_c + t) : 0.0;
-            }
-#pragma unroll
-            for (int k = 0; k < kChunk; ++k)
-                if (t0 + 32 * k + lane < cnt_c) buf[dd[k]] = lu_sub(buf[dd[k]], lu_mul(u, ll[k]));
-        }
-        __syncwarp();
-        have_c = have_n;
-        rd_c = rd_n;
-        lv_c = lv_n;
-        l0_c = l0_n;
-        cnt_c = cnt_n;
-        us_c = us_n;
-        ld_c = ld_n;
     }
+    timed_out = __shfl_sync(0xffffffffu, timed_out, 0);
     const double piv = buf[dj];
     ColumnResult res{kStatusOk, false, timed_out};
     if (amd) {
@@ -376,17 +439,25 @@ __device__ __forceinline__ ColumnResult refactor_column(
     } else {
         res.code = (piv == 0.0) ? kStatusSingular : kStatusOk;
     }
-    const int32_t* rowcopy = pool + pd.off[PA_rowcopy_pos];
+    // The column's values, then its completion: the row-major copies, which
+    // only the sweeps read, follow off the other columns' critical path.
+    const double inv = amd ? piv : 1.0 / piv;
     for (int32_t t = lane; t < len; t += 32) {
-        const double v = lu_store_value(amd, buf[t], t, dj, piv);
+        double v = buf[t];
+        if (amd ? t > dj : t == dj) v = amd ? __ddiv_rn(v, piv) : inv;
         lu[c0 + t] = v;
-        if (lrows) {
-            if (t < dj) urows[rowcopy[c0 + t]] = v;
-            else if (t > dj) lrows[rowcopy[c0 + t]] = v;
+        buf[t] = v;
+    }
+    __syncwarp();
+    publish(res);
+    if (lrows) {
+        const int32_t* rowcopy = pool + pd.off[PA_rowcopy_pos];
+        for (int32_t t = lane; t < len; t += 32) {
+            if (t < dj) urows[rowcopy[c0 + t]] = buf[t];
+            else if (t > dj) lrows[rowcopy[c0 + t]] = buf[t];
         }
     }
     __syncwarp();
-    return res;
 }
 
 // Dataflow refactor of one instance by the whole CTA (blockDim.x ==
@@ -404,20 +475,21 @@ __device__ __forceinline__ ColumnResult refactor_column(
 // __syncthreads().
 // When lrows/urows are given, every L and U entry is also written to its
 // position in the row-major copies the dataflow sweeps read.
-static __device__ __noinline__ RefactorResult cta_refactor_flow(const PlanDesc& pd, const int32_t* __restrict__ pool,
+template <int kPlan, int kDest>
+static __device__ __noinline__ RefactorResult cta_refactor_flow_as(const PlanDesc& pd, const int32_t* __restrict__ pool,
                                                    const double* __restrict__ a, double* __restrict__ lu,
                                                    double diag_gmin, int check_pivots,
                                                    double rel_threshold, double* smem, int colbuf,
-                                                   double* __restrict__ lrows = nullptr,
-                                                   double* __restrict__ urows = nullptr,
-                                                   int32_t* rmaps = nullptr,
-                                                   int64_t rmap_stride = 0) {
+                                                   double* __restrict__ lrows,
+                                                   double* __restrict__ urows, int32_t* rmaps,
+                                                   int64_t rmap_stride) {
     const int32_t n = pd.n;
-    const bool amd = pd.kind == kPlanAmdLu;
+    const bool amd = kPlan == kPlanAmdLu;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     double* buf = smem + warp * colbuf;
-    volatile int32_t* done = reinterpret_cast<volatile int32_t*>(smem + kFlowWarps * colbuf);
+    volatile int32_t* done =
+        reinterpret_cast<volatile int32_t*>(smem + (blockDim.x >> 5) * colbuf);
     int32_t* rmap = rmaps ? rmaps + warp * rmap_stride : nullptr;
 
     __shared__ int32_t s_next, s_timeout, s_growth;
@@ -437,16 +509,17 @@ static __device__ __noinline__ RefactorResult cta_refactor_flow(const PlanDesc& 
         if (lane == 0) j = atomicAdd(&s_next, 1);
         j = __shfl_sync(0xffffffffu, j, 0);
         if (j >= n) break;
-        const ColumnResult c = refactor_column<false>(
+        refactor_column<false, kPlan, kDest>(
             pd, pool, a, lu, diag_gmin, check_pivots, rel_threshold, j, buf, lrows, urows,
-            [&](int32_t r) { return flag_acquire(done + r); }, rmap);
-        if (lane == 0) {
-            if (c.timed_out) s_timeout = 1;
-            else if (c.code != kStatusOk) atomicMin(&s_fail, fail_key(j, c.code));
-            if (c.growth_fail) s_growth = 1;
-            flag_release(done + j, 1);
-        }
-        __syncwarp();
+            [&](int32_t r) { return flag_acquire(done + r); },
+            [&](const ColumnResult& c) {
+                if (lane != 0) return;
+                if (c.timed_out) s_timeout = 1;
+                else if (c.code != kStatusOk) atomicMin(&s_fail, fail_key(j, c.code));
+                if (c.growth_fail) s_growth = 1;
+                flag_release(done + j, 1);
+            },
+            rmap);
     }
     __syncthreads();
     RefactorResult res;
@@ -462,6 +535,31 @@ static __device__ __noinline__ RefactorResult cta_refactor_flow(const PlanDesc& 
     }
     __syncthreads();
     return res;
+}
+
+// The dataflow refactor compiled for the plan's engine and for the way its
+// update destinations are found (a column that fits shared memory has a packed
+// update map unless row maps were asked for).
+static __device__ __forceinline__ RefactorResult cta_refactor_flow(
+    const PlanDesc& pd, const int32_t* pool, const double* a, double* lu, double diag_gmin,
+    int check_pivots, double rel_threshold, double* smem, int colbuf, double* lrows = nullptr,
+    double* urows = nullptr, int32_t* rmaps = nullptr, int64_t rmap_stride = 0) {
+    if (pd.kind == kPlanAmdLu) {
+        if (rmaps)
+            return cta_refactor_flow_as<kPlanAmdLu, kDestRowMap>(
+                pd, pool, a, lu, diag_gmin, check_pivots, rel_threshold, smem, colbuf, lrows, urows,
+                rmaps, rmap_stride);
+        return cta_refactor_flow_as<kPlanAmdLu, kDestMap16>(
+            pd, pool, a, lu, diag_gmin, check_pivots, rel_threshold, smem, colbuf, lrows, urows,
+            nullptr, 0);
+    }
+    if (rmaps)
+        return cta_refactor_flow_as<kPlanMarkowitz, kDestRowMap>(
+            pd, pool, a, lu, diag_gmin, check_pivots, rel_threshold, smem, colbuf, lrows, urows,
+            rmaps, rmap_stride);
+    return cta_refactor_flow_as<kPlanMarkowitz, kDestMap16>(
+        pd, pool, a, lu, diag_gmin, check_pivots, rel_threshold, smem, colbuf, lrows, urows, nullptr,
+        0);
 }
 
 // x <- A^{-1} x (SparseMatrix::solve, or AmdLuSolver::solve,
@@ -539,11 +637,16 @@ __device__ inline void cta_solve(const PlanDesc& pd, const int32_t* __restrict__
 // small path) followed by an optional stage for instance workspaces, capped
 // so that two CTAs still fit on an SM.
 constexpr size_t kStageCapBytes = 100 * 1024;
-__host__ __device__ inline size_t stage_bytes_for(size_t scratch_bytes, long long max_stage) {
-    if (scratch_bytes >= kStageCapBytes || max_stage <= 0) return 0;
-    const size_t want = static_cast<size_t>(max_stage) * sizeof(double);
-    const size_t room = kStageCapBytes - scratch_bytes;
-    return want < room ? want : room;
+// lens: the instances' staged doubles, ascending.  The stage holds the largest
+// instance that fits, provided that half of the batch does: shared memory that
+// few instances use is better left to L1 (a batch of meshes too large for the
+// stage ran 1.4 times slower with the room reserved for it).
+inline size_t stage_bytes_for(size_t scratch_bytes, const int64_t* lens, int count) {
+    if (scratch_bytes >= kStageCapBytes || count <= 0) return 0;
+    const int64_t room = static_cast<int64_t>((kStageCapBytes - scratch_bytes) / sizeof(double));
+    int fit = 0;
+    while (fit < count && lens[fit] <= room) ++fit;
+    return 2 * fit >= count ? sizeof(double) * static_cast<size_t>(lens[fit - 1]) : 0;
 }
 
 __host__ __device__ inline bool small_fits(int n, int nnz_lu, int smem_doubles) {
@@ -829,7 +932,7 @@ static __device__ __noinline__ RefactorResult cta_refactor_small(
             }
             double colmax = 0.0;  // AMD-LU: largest |U(r, j)| applied (lane 0)
             for (int32_t q = 0; q < dj; ++q) {
-                const int4 m = umeta[c0 + q];  // r, diag_pos[r], |L(:, r)|, upd_start
+                const int4 m = u_entry(umeta, c0 + q);  // r, diag_pos[r], |L(:, r)|, upd_start
                 if (m.z <= kSmallSerialRows) {
                     if (lane == 0) {
                         const double u = amd ? lu_s[c0 + q] : lu_mul(lu_s[c0 + q], lu_s[m.y]);

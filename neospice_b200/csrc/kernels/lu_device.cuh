@@ -42,6 +42,15 @@ __device__ __forceinline__ int32_t upd_at(const int32_t* upd_dst, int32_t map16,
 }
 #endif
 
+#ifdef __CUDACC__
+// U entry q of a plan's umeta without its run bit (kRunBit of the third word).
+__device__ __forceinline__ int4 u_entry(const int4* umeta, int32_t q) {
+    int4 m = umeta[q];
+    m.z &= 0x7fffffff;
+    return m;
+}
+#endif
+
 struct InstDesc {
     int32_t plan;   // index into the PlanDesc array
     int32_t index;  // the instance's position in the caller's arrays

@@ -167,7 +167,7 @@ __device__ ColumnResult refactor_column_cta(const PlanDesc& pd, const int32_t* _
         off = static_cast<int>((reinterpret_cast<uintptr_t>(lu + l0) >> 3) & 1);
     };
     auto stage = [&](int32_t q) {
-        const int4 m = umeta[q];
+        const int4 m = u_entry(umeta, q);
         const int slot = q % kCtaRing;
         int32_t l0, ns;
         int off;
@@ -224,7 +224,7 @@ __device__ ColumnResult refactor_column_cta(const PlanDesc& pd, const int32_t* _
         }
         cp_async_wait(staged - q - 1);
         __syncthreads();
-        const int4 m = umeta[q];
+        const int4 m = u_entry(umeta, q);
         const int slot = q % kCtaRing;
         int32_t l0, ns;
         int off;
@@ -315,18 +315,19 @@ grid_refactor_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restri
         const int32_t len = col_ptr[j + 1] - col_ptr[j];
         double* buf = (len <= kColbuf) ? sbuf : lu + col_ptr[j];
         auto probe = [&](int32_t r) { return gflag_acquire(done + r); };
-        const ColumnResult c = refactor_column<true, decltype(probe), kGridChunk>(
+        refactor_column<true, -1, -1, kGridChunk>(
             pd, pool, A + id.a_off, lu, diag_gmin, check_pivots, rel_threshold, j, buf, lr, ur,
-            probe, rmap);
-        __threadfence();
-        __syncwarp();
-        if (lane == 0) {
-            if (c.timed_out) atomicExch(&st->timeout, 1);
-            else if (c.code != kStatusOk) atomicMax(&st->fail_inv, ~fail_key(j, c.code));
-            if (c.growth_fail) atomicExch(&st->growth, 1);
-            gflag_release(done + j, 1);
-        }
-        __syncwarp();
+            probe,
+            [&](const ColumnResult& c) {
+                __threadfence();
+                __syncwarp();
+                if (lane != 0) return;
+                if (c.timed_out) atomicExch(&st->timeout, 1);
+                else if (c.code != kStatusOk) atomicMax(&st->fail_inv, ~fail_key(j, c.code));
+                if (c.growth_fail) atomicExch(&st->growth, 1);
+                gflag_release(done + j, 1);
+            },
+            rmap);
     }
     if constexpr (kColbuf >= 2048) {
         if (warp_end < pd.n) {

@@ -12,11 +12,12 @@
 
 namespace nsg {
 
-// Two CTAs per SM: registers are capped at 64 per thread.  subset (optional)
+// kBlocks CTAs of kThreads threads per SM.  subset (optional)
 // lists the descriptor positions to run, one per block.  ctls[index] is the
 // instance's operating-point controller: zeroed by the host for a fresh run,
 // kept across launches when an instance stopped with kStatusReorder.
-__global__ void __launch_bounds__(kFlowThreads, 2)
+template <int kThreads, int kBlocks>
+__global__ void __launch_bounds__(kThreads, kBlocks)
 newton_dc_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restrict__ lu_pool,
                  const DcDesc* __restrict__ descs, const int32_t* __restrict__ subset,
                  const int32_t* __restrict__ prog, const double* __restrict__ params,
@@ -38,9 +39,9 @@ newton_dc_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restrict__
     // dataflow scratch of large meshes fills the shared memory of two CTAs
     // per SM to within a few hundred bytes.
     Inst v = make_inst(d, prog, params, work, stage);
-    static_assert(kFlowWarps == 16, "the host sizes the row maps for 16 warps per CTA");
+    static_assert(kThreads <= 32 * kDcMaxWarps, "the host sizes the row maps for kDcMaxWarps");
     if (rmaps) {
-        v.rmaps = rmaps + static_cast<int64_t>(blockIdx.x) * kFlowWarps * rmap_stride;
+        v.rmaps = rmaps + static_cast<int64_t>(blockIdx.x) * kDcMaxWarps * rmap_stride;
         v.rmap_stride = rmap_stride;
     }
     __shared__ IntegCtx ctx;
@@ -79,45 +80,77 @@ newton_dc_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restrict__
     }
 }
 
-size_t dc_smem_bytes(int max_col, int max_n) {
+namespace {
+
+size_t dc_scratch_bytes(int max_col, int max_n, int warps) {
     const int colbuf = (max_col + 31) & ~31;
-    const size_t a = flow_smem_bytes(colbuf, max_n);
+    const size_t a = flow_smem_bytes(colbuf, max_n, warps);
     const size_t b = flow_solve_smem_bytes(max_n);
     return a > b ? a : b;
 }
 
+template <int kThreads, int kBlocks>
+cudaError_t configure_dc() {
+    static const cudaError_t e =
+        cudaFuncSetAttribute(newton_dc_kernel<kThreads, kBlocks>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    return e;
+}
+
+int dc_sm_count() {
+    static const int sms = [] {
+        int dev = 0, n = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        return n > 0 ? n : 1;
+    }();
+    return sms;
+}
+
+}  // namespace
+
+size_t dc_smem_bytes(int max_col, int max_n) {
+    return dc_scratch_bytes(max_col, max_n, kFlowWarps);
+}
+
+// Launch shape: up to one instance per SM, one CTA of 24 warps has the SM's
+// registers (80 a thread) to itself; more instances run as CTAs of 16 warps,
+// two per SM (64 registers).  One 2305-unknown mesh took 12.8 ms with the
+// first and 16.3 ms with the second shape, 148 of 5185 unknowns 41.7 and
+// 55.0 ms, 600 of 257 to 1601 unknowns 18.1 and 14.1 ms.  stage_lens: the
+// instances' stage_len, ascending.
 cudaError_t launch_newton_dc(const PlanDesc* plans, const int32_t* lu_pool, const DcDesc* descs,
                              const int32_t* subset, int count, const int32_t* prog,
                              const double* params, double* work, double* solutions,
                              int32_t* status, int32_t* iterations, DcCtl* ctls,
                              const NewtonOptions& opt, int max_col, int max_n,
-                             long long max_stage, int lp_doubles, int plan_words,
-                             int32_t* rmaps, cudaStream_t stream) {
+                             const int64_t* stage_lens, int n_stage, int lp_doubles,
+                             int plan_words, int32_t* rmaps, cudaStream_t stream) {
     if (count <= 0) return cudaSuccess;
     const int colbuf = (max_col + 31) & ~31;
+    const bool wide = count <= dc_sm_count() &&
+                      dc_scratch_bytes(max_col, max_n, kDcMaxWarps) <= 200 * 1024;
     const size_t level = sizeof(double) * static_cast<size_t>(lp_doubles);
-    const size_t flow = dc_smem_bytes(max_col, max_n);
+    const size_t flow = dc_scratch_bytes(max_col, max_n, wide ? kDcMaxWarps : kFlowWarps);
     const size_t scratch = ((flow > level ? flow : level) + 15) & ~size_t{15};
     size_t plan = (sizeof(int32_t) * static_cast<size_t>(plan_words) + 15) & ~size_t{15};
     if (scratch + plan > kStageCapBytes) plan = 0;  // read from global memory instead
-    const size_t stage = stage_bytes_for(scratch + plan, max_stage);
+    const size_t stage = stage_bytes_for(scratch + plan, stage_lens, n_stage);
     const size_t smem = scratch + stage + plan;
     if (smem > 200 * 1024) return cudaErrorInvalidValue;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(newton_dc_kernel,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             200 * 1024);
-        if (e != cudaSuccess) return e;
-        configured = true;
-    }
-    newton_dc_kernel<<<count, kFlowThreads, smem, stream>>>(plans, lu_pool, descs, subset, prog,
-                                                             params, work, solutions, status,
-                                                             iterations, ctls, opt, colbuf,
-                                                             static_cast<int>(scratch / sizeof(double)),
-                                                             static_cast<int>(stage / sizeof(double)),
-                                                             static_cast<int>(plan / sizeof(int32_t)),
-                                                             rmaps, max_n);
+    const int scratch_d = static_cast<int>(scratch / sizeof(double));
+    const int stage_d = static_cast<int>(stage / sizeof(double));
+    const int plan_w = static_cast<int>(plan / sizeof(int32_t));
+    const cudaError_t e = wide ? configure_dc<32 * kDcMaxWarps, 1>() : configure_dc<kFlowThreads, 2>();
+    if (e != cudaSuccess) return e;
+    if (wide)
+        newton_dc_kernel<32 * kDcMaxWarps, 1><<<count, 32 * kDcMaxWarps, smem, stream>>>(
+            plans, lu_pool, descs, subset, prog, params, work, solutions, status, iterations, ctls,
+            opt, colbuf, scratch_d, stage_d, plan_w, rmaps, max_n);
+    else
+        newton_dc_kernel<kFlowThreads, 2><<<count, kFlowThreads, smem, stream>>>(
+            plans, lu_pool, descs, subset, prog, params, work, solutions, status, iterations, ctls,
+            opt, colbuf, scratch_d, stage_d, plan_w, rmaps, max_n);
     return cudaGetLastError();
 }
 

@@ -3,6 +3,7 @@
 #include "dc_device.cuh"
 
 #include <cstdint>
+#include <vector>
 
 namespace nsg {
 
@@ -59,13 +60,13 @@ struct TranCtl {
 };
 
 // What the launch needs to size one CTA: the batch's largest LU column and
-// unknown count (dataflow scratch), largest staged workspace, largest
+// unknown count (dataflow scratch), the instances' staged workspaces, largest
 // shared-memory LU (doubles: nnz_lu + n, or a level program's space), largest
 // space of a level program, most words of a plan to keep in shared memory and
 // most devices of one family in one instance (the device loads' parallelism).
 struct TranShape {
     int32_t max_col, max_n;
-    int64_t max_stage;
+    std::vector<int64_t> stage_lens;  // ascending
     int32_t max_small_lu;
     int32_t lp_doubles;
     int32_t plan_words;

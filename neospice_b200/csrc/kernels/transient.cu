@@ -578,7 +578,8 @@ cudaError_t launch_transient(const PlanDesc* plans, const int32_t* lu_pool, cons
         scratch = ((flow > level ? flow : level) + 15) & ~size_t{15};
         plan = (sizeof(int32_t) * static_cast<size_t>(sh.plan_words) + 15) & ~size_t{15};
         if (scratch + plan > kStageCapBytes) plan = 0;  // read from global memory instead
-        stage = stage_bytes_for(scratch + plan, sh.max_stage);
+        stage = stage_bytes_for(scratch + plan, sh.stage_lens.data(),
+                                static_cast<int>(sh.stage_lens.size()));
     } else {
         // Per-CTA share of the SM's 228 KB, less the CTA's static shared
         // memory and the 1 KB the runtime reserves per CTA.
@@ -586,7 +587,7 @@ cudaError_t launch_transient(const PlanDesc* plans, const int32_t* lu_pool, cons
         scratch = (sizeof(double) * static_cast<size_t>(sh.max_small_lu) + 15) & ~size_t{15};
         plan = (sizeof(int32_t) * static_cast<size_t>(sh.plan_words) + 15) & ~size_t{15};
         if (scratch + plan > budget) plan = 0;
-        const size_t want = static_cast<size_t>(sh.max_stage) * sizeof(double);
+        const size_t want = static_cast<size_t>(sh.stage_lens.back()) * sizeof(double);
         stage = (scratch + plan + want <= budget) ? want : 0;
     }
     const size_t smem = scratch + stage + plan;
