@@ -34,10 +34,12 @@ cudaError_t launch_grid_refactor(const PlanDesc* plans, const int32_t* pool,
                                  const int32_t* cta_from_of, cudaStream_t stream);
 int64_t grid_rmap_words(int colbuf, int max_col, int max_n);
 cudaError_t launch_complex_refactor(const PlanDesc* plans, const int32_t* pool,
-                                    const InstDesc* insts, int count, int max_n, const double* A,
-                                    double* LU, int32_t* status, cudaStream_t stream);
+                                    const InstDesc* insts, int count, int max_col, int max_n,
+                                    const double* A, double* LU, int32_t* status,
+                                    cudaStream_t stream);
+bool complex_solve_in_smem(int max_n, const double* LU);
 cudaError_t launch_complex_solve(const PlanDesc* plans, const int32_t* pool, const InstDesc* insts,
-                                 int count, const double* LU, double* X, double* W,
+                                 int count, int max_n, const double* LU, double* X, double* W,
                                  cudaStream_t stream);
 size_t complex_refactor_smem(int max_n);
 cudaError_t launch_grid_solve(const PlanDesc* plans, const int32_t* pool, const InstDesc* insts,
@@ -595,7 +597,7 @@ int nsg_batch_refactor_complex(nsg_batch* b, const double* d_ax, double* d_lu, i
         return fail(NSG_ERR_INVALID, "nsg_batch_refactor_complex: too many unknowns per instance "
                                      "for the shared-memory completion flags");
     const cudaError_t e = nsg::launch_complex_refactor(b->d_plans, b->d_pool, b->d_insts, b->count,
-                                                       b->max_n, d_ax, d_lu, d_status,
+                                                       b->max_col, b->max_n, d_ax, d_lu, d_status,
                                                        static_cast<cudaStream_t>(stream));
     return e == cudaSuccess ? NSG_OK : cuda_fail("nsg_batch_refactor_complex", e);
 }
@@ -603,12 +605,12 @@ int nsg_batch_refactor_complex(nsg_batch* b, const double* d_ax, double* d_lu, i
 int nsg_batch_solve_complex(nsg_batch* b, const double* d_lu, double* d_x, void* stream) {
     if (!b || !d_lu || !d_x) return fail(NSG_ERR_INVALID, "nsg_batch_solve_complex: null argument");
     cudaError_t e = cudaSuccess;
-    if (!b->d_cwork) {
+    if (!b->d_cwork && !nsg::complex_solve_in_smem(b->max_n, d_lu)) {
         e = cudaMalloc(reinterpret_cast<void**>(&b->d_cwork),
                        sizeof(double) * 2 * static_cast<size_t>(std::max<long long>(1, b->x_off[b->count])));
         if (e != cudaSuccess) return cuda_fail("nsg_batch_solve_complex: workspace", e);
     }
-    e = nsg::launch_complex_solve(b->d_plans, b->d_pool, b->d_insts, b->count, d_lu, d_x,
+    e = nsg::launch_complex_solve(b->d_plans, b->d_pool, b->d_insts, b->count, b->max_n, d_lu, d_x,
                                   b->d_cwork, static_cast<cudaStream_t>(stream));
     return e == cudaSuccess ? NSG_OK : cuda_fail("nsg_batch_solve_complex", e);
 }
