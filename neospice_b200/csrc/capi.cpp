@@ -43,9 +43,9 @@ cudaError_t launch_complex_solve(const PlanDesc* plans, const int32_t* pool, con
                                  cudaStream_t stream);
 size_t complex_refactor_smem(int max_n);
 cudaError_t launch_grid_solve(const PlanDesc* plans, const int32_t* pool, const InstDesc* insts,
-                              int count, const int32_t* n_of, const double* LU,
-                              const double* lrows, const double* urows, double* X, double* W,
-                              void* scratch, cudaStream_t stream);
+                              int count, const int32_t* n_of, int max_n, const double* LU,
+                              const double* lrows, const double* urows, double* X, void* scratch,
+                              cudaStream_t stream);
 }  // namespace nsg
 
 namespace nsg {
@@ -674,8 +674,8 @@ int nsg_batch_solve(nsg_batch* b, double* d_x, void* stream) {
     if (!b || !d_x) return fail(NSG_ERR_INVALID, "nsg_batch_solve: null argument");
     if (b->schedule == 2 && b->rows_valid && b->d_grid) {
         cudaError_t e = nsg::launch_grid_solve(b->d_plans, b->d_pool, b->d_insts, b->count,
-                                               b->n_of.data(), b->d_lu, b->d_lrows, b->d_urows,
-                                               d_x, b->d_work, b->d_grid,
+                                               b->n_of.data(), b->max_n, b->d_lu, b->d_lrows,
+                                               b->d_urows, d_x, b->d_grid,
                                                static_cast<cudaStream_t>(stream));
         return e == cudaSuccess ? NSG_OK : cuda_fail("nsg_batch_solve", e);
     }
