@@ -320,19 +320,97 @@ static __device__ __noinline__ void eval_devices(const Inst& v, const IntegCtx& 
     }
 }
 
-// Matrix values and rhs (into x) from the stamp program, in load order.
-__device__ inline void assemble(const Inst& v) {
-    for (int32_t s = threadIdx.x; s < v.nnz; s += blockDim.x) {
-        double acc = 0.0;
-        for (int32_t k = v.slot_ptr[s]; k < v.slot_ptr[s + 1]; ++k)
-            acc = __dadd_rn(acc, v.tv[v.slot_terms[k]]);
-        v.a[s] = acc;
+// Sum of tv over terms[b .. e - 1], one after another.  The indices and values
+// are loaded kAsmChunk at a time ahead of the adds, which take them in order; a
+// missing one adds +0.0, which changes no sum that starts from +0.0.
+constexpr int kAsmChunk = 8;
+__device__ __forceinline__ double sum_terms(const int32_t* terms, int32_t b, int32_t e,
+                                            const double* tv) {
+    double acc = 0.0;
+    for (int32_t k = b; k < e; k += kAsmChunk) {
+        int32_t at[kAsmChunk];
+        double x[kAsmChunk];
+#pragma unroll
+        for (int u = 0; u < kAsmChunk; ++u) at[u] = k + u < e ? terms[k + u] : -1;
+#pragma unroll
+        for (int u = 0; u < kAsmChunk; ++u) x[u] = at[u] >= 0 ? tv[at[u]] : 0.0;
+#pragma unroll
+        for (int u = 0; u < kAsmChunk; ++u) acc = __dadd_rn(acc, x[u]);
     }
-    for (int32_t i = threadIdx.x; i < v.n; i += blockDim.x) {
-        double nat = 0.0, ucb = 0.0;
-        for (int32_t k = v.rhs_ptr[i]; k < v.rhs_ptr[i + 1]; ++k) nat = __dadd_rn(nat, v.tv[v.rhs_terms[k]]);
-        for (int32_t k = v.ucb_ptr[i]; k < v.ucb_ptr[i + 1]; ++k) ucb = __dadd_rn(ucb, v.tv[v.ucb_terms[k]]);
-        v.x[i] = __dadd_rn(nat, ucb);
+    return acc;
+}
+
+// The same by a whole warp: 32 indices and values at once (the next 32 in
+// flight), the adds in order in every lane.
+__device__ __forceinline__ double sum_terms_warp(const int32_t* terms, int32_t b, int32_t e,
+                                                 const double* tv) {
+    const int lane = threadIdx.x & 31;
+    double acc = 0.0;
+    int32_t at = b + lane < e ? terms[b + lane] : -1;
+    double x = at >= 0 ? tv[at] : 0.0;
+    at = b + 32 + lane < e ? terms[b + 32 + lane] : -1;
+    for (int32_t k = b; k < e; k += 32) {
+        const double cur = x;
+        x = at >= 0 ? tv[at] : 0.0;
+        at = k + 64 + lane < e ? terms[k + 64 + lane] : -1;
+        const int32_t m = min(32, e - k);
+        int32_t u = 0;
+        for (; u + 4 <= m; u += 4) {
+            const double p0 = __shfl_sync(0xffffffffu, cur, u);
+            const double p1 = __shfl_sync(0xffffffffu, cur, u + 1);
+            const double p2 = __shfl_sync(0xffffffffu, cur, u + 2);
+            const double p3 = __shfl_sync(0xffffffffu, cur, u + 3);
+            acc = __dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(acc, p0), p1), p2), p3);
+        }
+        for (; u < m; ++u) acc = __dadd_rn(acc, __shfl_sync(0xffffffffu, cur, u));
+    }
+    return acc;
+}
+
+// Matrix values and rhs (into x) from the stamp program, in load order: a thread
+// per matrix slot or rhs row, the rows beside the slots.  Lists longer than
+// kAsmLong (a supply node's, with terms of every device on it) are summed by
+// the whole warp, one after another.  One load after another, a thread took
+// two memory round trips a term: 400 inverter chains 55.0 -> 51.5 ms, 300
+// BSIM4v7 ring + NAND instances 108 -> 99 ms.
+constexpr int32_t kAsmLong = 24;
+static __device__ __noinline__ void assemble(const Inst& v) {
+    const int lane = threadIdx.x & 31;
+    const int32_t total = v.nnz + v.n;
+    for (int32_t s0 = threadIdx.x - lane; s0 < total; s0 += blockDim.x) {
+        const int32_t s = s0 + lane;
+        // list b .. e - 1 of the slot terms (slots) or rhs terms (rows), and
+        // rows' second list in the UCB terms
+        int32_t b = 0, e = 0, b2 = 0, e2 = 0;
+        if (s < v.nnz) {
+            b = v.slot_ptr[s];
+            e = v.slot_ptr[s + 1];
+        } else if (s < total) {
+            b = v.rhs_ptr[s - v.nnz];
+            e = v.rhs_ptr[s - v.nnz + 1];
+            b2 = v.ucb_ptr[s - v.nnz];
+            e2 = v.ucb_ptr[s - v.nnz + 1];
+        }
+        const bool row = s >= v.nnz;
+        const bool lng = e - b > kAsmLong || e2 - b2 > kAsmLong;
+        double acc = 0.0;
+        if (!lng) {
+            acc = sum_terms(row ? v.rhs_terms : v.slot_terms, b, e, v.tv);
+            if (row) acc = __dadd_rn(acc, sum_terms(v.ucb_terms, b2, e2, v.tv));
+        }
+        for (unsigned mask = __ballot_sync(0xffffffffu, lng); mask; mask &= mask - 1) {
+            const int k = __ffs(mask) - 1;
+            const bool krow = s0 + k >= v.nnz;
+            double x = sum_terms_warp(krow ? v.rhs_terms : v.slot_terms,
+                                      __shfl_sync(0xffffffffu, b, k),
+                                      __shfl_sync(0xffffffffu, e, k), v.tv);
+            if (krow)
+                x = __dadd_rn(x, sum_terms_warp(v.ucb_terms, __shfl_sync(0xffffffffu, b2, k),
+                                                __shfl_sync(0xffffffffu, e2, k), v.tv));
+            if (lane == k) acc = x;
+        }
+        if (!row) v.a[s] = acc;
+        else if (s < total) v.x[s - v.nnz] = acc;
     }
 }
 
