@@ -165,9 +165,11 @@ NSG_HD inline void b4_overlap(double vx, double cgxo, double weffcv, double cgxl
 // voltages d, g, s, b of the previous iterate (0 for ground); reltol /
 // abstol: the convergence test's tolerances; t: the kBsim4Terms stamp
 // values.  rec[kB4RNoncon] receives 1 when the instance is not converged.
-NSG_HD inline void bsim4_load(const double* P, double* rec, double* s0, double* s1,
-                              const double* s2, int mode, const Mos1Integ& ic, double gmin,
-                              double reltol, double abstol, const double v[4], double* t) {
+NSG_HD inline void bsim4_load(const double* __restrict__ P, double* __restrict__ rec,
+                              double* __restrict__ s0, double* __restrict__ s1,
+                              const double* __restrict__ s2, int mode, const Mos1Integ& ic,
+                              double gmin, double reltol, double abstol, const double v[4],
+                              double* __restrict__ t) {
     const double type = P[kB4Type];
     const bool off = P[kB4Off] != 0.0;
     const bool charge =

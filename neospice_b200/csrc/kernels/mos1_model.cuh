@@ -237,9 +237,10 @@ NSG_HD inline void m1_bulk_charge(const double* P, double v, bool drain, double*
 // instance values; s0/s1/s2: the instance's state slots in the state ring;
 // v[4]: node voltages d, g, s, b of the previous iterate (0 for ground);
 // t: the kMos1Terms stamp values written in MOS1load's order.
-NSG_HD inline void mos1_load(const double* P, double* rec, double* s0, double* s1,
-                             const double* s2, int mode, const Mos1Integ& ic, double gmin,
-                             const double v[4], double* t) {
+NSG_HD inline void mos1_load(const double* __restrict__ P, double* __restrict__ rec,
+                             double* __restrict__ s0, double* __restrict__ s1,
+                             const double* __restrict__ s2, int mode, const Mos1Integ& ic,
+                             double gmin, const double v[4], double* __restrict__ t) {
     const double type = P[kMType];
     const double vt = P[kMVt];
     const double m = P[kMM];

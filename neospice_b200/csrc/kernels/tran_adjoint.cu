@@ -335,7 +335,8 @@ __device__ __noinline__ void mos_charge_update(const Inst& v, int32_t base, cons
 
 }  // namespace
 
-__global__ void __launch_bounds__(kFlowThreads, 2)
+template <int kBlocks>
+__global__ void __launch_bounds__(kFlowThreads, kBlocks)
 tran_adjoint_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restrict__ lu_pool,
                     const DcDesc* __restrict__ descs, const TranDesc* __restrict__ tdescs,
                     const AdjDesc* __restrict__ adescs, const int32_t* __restrict__ prog,
@@ -723,19 +724,24 @@ cudaError_t launch_tran_adjoint(const PlanDesc* plans, const int32_t* lu_pool, c
     if (scratch + plan > kStageCapBytes) plan = 0;  // read from global memory instead
     const size_t smem = scratch + plan;
     if (smem > 200 * 1024) return cudaErrorInvalidValue;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(tran_adjoint_kernel,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             200 * 1024);
+    static const int sms = [] {
+        int dev = 0, n = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        return n > 0 ? n : 1;
+    }();
+    auto launch = [&](auto kernel) -> cudaError_t {
+        const cudaError_t e = cudaFuncSetAttribute(
+            kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         if (e != cudaSuccess) return e;
-        configured = true;
-    }
-    tran_adjoint_kernel<<<count, kFlowThreads, smem, stream>>>(
-        plans, lu_pool, descs, tdescs, adescs, prog, params_dc, params_tran, work, adj_ws, recs,
-        times, rec_x0, targets, weight, grads, loss, status, opt, max_iter, colbuf,
-        static_cast<int>(scratch / sizeof(double)), static_cast<int>(plan / sizeof(int32_t)));
-    return cudaGetLastError();
+        kernel<<<count, kFlowThreads, smem, stream>>>(
+            plans, lu_pool, descs, tdescs, adescs, prog, params_dc, params_tran, work, adj_ws, recs,
+            times, rec_x0, targets, weight, grads, loss, status, opt, max_iter, colbuf,
+            static_cast<int>(scratch / sizeof(double)), static_cast<int>(plan / sizeof(int32_t)));
+        return cudaGetLastError();
+    };
+    // one instance per SM has its registers (128 a thread) to itself
+    return count <= sms ? launch(tran_adjoint_kernel<1>) : launch(tran_adjoint_kernel<2>);
 }
 
 }  // namespace nsg

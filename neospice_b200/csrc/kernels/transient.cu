@@ -539,16 +539,20 @@ int sm_count() {
 
 }  // namespace
 
-// Launch shapes.  Latency of one instance is the cost for a few hundred
-// instances: one 512-thread CTA per instance, two per SM, each staging its
-// plan and workspace in shared memory.  When every instance takes the
-// shared-memory LU path (n <= 128) and the batch is larger than those two
-// CTAs per SM can hold at once, throughput is the cost: CTAs of 128 or 256
-// threads (as many as the instances' largest device family needs for one
-// pass of the device loads), eight or four per SM, with the LU and the plan
-// in shared memory and the workspace staged only where it fits.  (Two
-// 256-thread CTAs per SM at 128 registers spill less in the BSIM4v7 loads
-// but ran 20 % slower than four at 64 on the ring + NAND Monte Carlo.)
+// Launch shapes.  The device loads are long serial chains of one thread each,
+// and at 64 registers a thread they spill; so CTAs are as small as the loads
+// need for one pass, and get as many registers as the instances in flight
+// leave.  When every instance is small (n <= 128):
+//   up to one instance per SM   one CTA of 256 threads (255 registers)
+//   more                        CTAs of 128 or 256 threads, as many as the
+//                               largest device family needs (128 registers):
+//                               four or two per SM
+// else CTAs of 512 threads, one per SM (128 registers) or two (64).
+// Passes measured on a B200, two CTAs of 512 threads per SM (small batches) or
+// 1024 threads per SM (large ones) -> these: one inverter chain 25.8 -> 20.4
+// ms, 400 chains 37.3 -> 35.4, 1184 chains 94.7 -> 94.3; BSIM4v7 ring + NAND,
+// 300 instances 79.3 -> 69.2, 1184 instances 224 -> 197 ms; transient and
+// adjoint of 64 500-node trees 32.9 -> 27.9 ms.
 // sh.force_threads / force_blocks (0: automatic) override the choice.
 cudaError_t launch_transient(const PlanDesc* plans, const int32_t* lu_pool, const DcDesc* descs,
                              const TranDesc* tdescs, const int32_t* subset, int count,
@@ -560,10 +564,11 @@ cudaError_t launch_transient(const PlanDesc* plans, const int32_t* lu_pool, cons
                              StepRecord* rec_steps, double* rec_x0, cudaStream_t stream) {
     if (count <= 0) return cudaSuccess;
     const int colbuf = (sh.max_col + 31) & ~31;
-    int threads = kFlowThreads, blocks = 2;
-    if (sh.max_n <= 128 && count > 2 * sm_count()) {
-        threads = sh.max_devices <= 128 ? 128 : (sh.max_devices <= 256 ? 256 : kFlowThreads);
-        blocks = threads == 128 ? 8 : (threads == 256 ? 4 : 2);
+    const bool alone = count <= sm_count();
+    int threads = kFlowThreads, blocks = alone ? 1 : 2;
+    if (sh.max_n <= 128 && sh.max_devices <= 256) {
+        threads = (alone || sh.max_devices > 128) ? 256 : 128;
+        blocks = alone ? 1 : 512 / threads;
     }
     if (sh.force_threads > 0) {
         threads = sh.force_threads;
@@ -582,8 +587,10 @@ cudaError_t launch_transient(const PlanDesc* plans, const int32_t* lu_pool, cons
                                 static_cast<int>(sh.stage_lens.size()));
     } else {
         // Per-CTA share of the SM's 228 KB, less the CTA's static shared
-        // memory and the 1 KB the runtime reserves per CTA.
-        const size_t budget = (228 * 1024) / static_cast<size_t>(blocks) - 3 * 1024;
+        // memory and the 1 KB the runtime reserves per CTA; the rest of a
+        // larger share is better left to L1.
+        const size_t share = (228 * 1024) / static_cast<size_t>(blocks) - 3 * 1024;
+        const size_t budget = share < kStageCapBytes ? share : kStageCapBytes;
         scratch = (sizeof(double) * static_cast<size_t>(sh.max_small_lu) + 15) & ~size_t{15};
         plan = (sizeof(int32_t) * static_cast<size_t>(sh.plan_words) + 15) & ~size_t{15};
         if (scratch + plan > budget) plan = 0;
@@ -602,12 +609,20 @@ cudaError_t launch_transient(const PlanDesc* plans, const int32_t* lu_pool, cons
         plans, lu_pool, descs, tdescs, subset, prog, params_dc, params_tran, work, bps, probes, \
         times, values, npoints, status, stats, ctls, o, colbuf, scratch_d, stage_d, rec_steps,  \
         rec_x0, plan_w);
-    if (threads == 128 && blocks == 8) {
-        NSG_LAUNCH_TRAN(128, 8)
-    } else if (threads == 256 && blocks == 4) {
-        NSG_LAUNCH_TRAN(256, 4)
+    if (threads == 128 && blocks == 4) {
+        NSG_LAUNCH_TRAN(128, 4)
+    } else if (threads == 256 && blocks == 2) {
+        NSG_LAUNCH_TRAN(256, 2)
+    } else if (threads == 256 && blocks == 1) {
+        NSG_LAUNCH_TRAN(256, 1)
+    } else if (threads == kFlowThreads && blocks == 1) {
+        NSG_LAUNCH_TRAN(kFlowThreads, 1)
     } else if (threads == kFlowThreads && blocks == 2) {
         NSG_LAUNCH_TRAN(kFlowThreads, 2)
+    } else if (threads == 128 && blocks == 8) {  // asked for (nsg_tran_batch_set_shape)
+        NSG_LAUNCH_TRAN(128, 8)
+    } else if (threads == 256 && blocks == 4) {  // asked for
+        NSG_LAUNCH_TRAN(256, 4)
     } else {
         return cudaErrorInvalidValue;
     }
