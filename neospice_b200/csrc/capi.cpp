@@ -4,6 +4,7 @@
 #include "kernels/dc_device.cuh"
 
 #include <algorithm>
+#include <atomic>
 #include <cstdlib>
 #include <cstring>
 #include <exception>
@@ -11,6 +12,7 @@
 #include <new>
 #include <stdexcept>
 #include <string>
+#include <thread>
 #include <unordered_map>
 #include <vector>
 
@@ -236,9 +238,32 @@ int intern_topology(std::vector<std::unique_ptr<nsg_topology>>& topos,
                     std::unique_ptr<nsg_topology> t) {
     for (size_t k = 0; k < topos.size(); ++k)
         if (same_plan(topos[k]->plan, t->plan)) return static_cast<int>(k);
-    nsg::build_level_program(t->plan);
     topos.push_back(std::move(t));
     return static_cast<int>(topos.size()) - 1;
+}
+
+void build_programs(std::vector<std::unique_ptr<nsg_topology>>& topos, size_t from) {
+    const size_t count = topos.size() > from ? topos.size() - from : 0;
+    std::atomic<size_t> next{from};
+    std::vector<std::exception_ptr> errs(count);
+    auto work = [&] {
+        for (size_t k; (k = next.fetch_add(1)) < topos.size();) try {
+                nsg::build_level_program(topos[k]->plan);
+            } catch (...) {
+                errs[k - from] = std::current_exception();
+            }
+    };
+    const size_t threads =
+        std::min<size_t>(count / 4, std::max(1u, std::thread::hardware_concurrency()));
+    if (threads <= 1) {
+        work();
+    } else {
+        std::vector<std::thread> pool;
+        for (size_t t = 0; t < threads; ++t) pool.emplace_back(work);
+        for (auto& th : pool) th.join();
+    }
+    for (auto& e : errs)
+        if (e) std::rethrow_exception(e);
 }
 
 int reorder_instance(std::vector<std::unique_ptr<nsg_topology>>& topos, int topo,

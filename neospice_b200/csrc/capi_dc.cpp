@@ -526,11 +526,11 @@ int nsg_dc_batch_create(int count, nsg_circuit* const* circuits, int symbolic, i
                 }
             if (topo_of[i] < 0) {
                 topo_of[i] = static_cast<int>(b->topos.size());
-                nsg::build_level_program(ordered[i]->plan);
                 b->topos.push_back(std::move(ordered[i]));
             }
         }
         for (int i = 0; i < count; ++i) topo_of[i] = topo_of[rep[i]];
+        build_programs(b->topos, 0);
 
         // Device plans, programs, descriptors, workspace.
         std::vector<int32_t> lu_pool, prog;
@@ -803,6 +803,7 @@ int nsg_dc_batch_run(nsg_dc_batch* b, const double* d_params, double* d_solution
                                 cudaMemcpyDeviceToHost)) != cudaSuccess)
                 return cuda_fail("nsg_dc_batch_run", e);
             std::vector<int32_t> subset;
+            const size_t ntopos = b->topos.size();
             for (int i = 0; i < b->count; ++i) {
                 if (status[i] != NSG_REORDER) continue;
                 nsg::DcDesc& d = b->descs[b->desc_pos[i]];
@@ -824,6 +825,7 @@ int nsg_dc_batch_run(nsg_dc_batch* b, const double* d_params, double* d_solution
                 ++b->reorders;
             }
             if (subset.empty()) break;
+            build_programs(b->topos, ntopos);
             b->drop_graph();  // plans and workspace move
             int rc = refresh_plans(b->topos, &b->d_lu_pool, &b->d_plans, &b->max_col, &b->max_n);
             if (rc != NSG_OK) return rc;

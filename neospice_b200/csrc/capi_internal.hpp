@@ -155,6 +155,9 @@ std::unique_ptr<nsg_topology> clone_topology(const nsg_topology& t);
 bool same_plan(const nsg::TopologyPlan& a, const nsg::TopologyPlan& b);
 int intern_topology(std::vector<std::unique_ptr<nsg_topology>>& topos,
                     std::unique_ptr<nsg_topology> t);
+// The level programs of topos[from ..] (the topologies a caller has just added),
+// on the host's threads.
+void build_programs(std::vector<std::unique_ptr<nsg_topology>>& topos, size_t from);
 int reorder_instance(std::vector<std::unique_ptr<nsg_topology>>& topos, int topo,
                      const double* values, double diag_gmin, int* new_topo);
 // Fresh LU / row-copy regions for a re-ordered instance at the end of the

@@ -241,6 +241,7 @@ int nsg_tran_batch_create(int count, nsg_circuit* const* circuits, double tstep,
                                           "instance " + std::to_string(i));
         std::vector<int> plan_dc(count);
         for (int i = 0; i < count; ++i) plan_dc[i] = intern_topology(b->topos, std::move(ord_dc[i]));
+        build_programs(b->topos, 0);
 
         std::vector<int32_t> lu_pool, prog;
         std::vector<nsg::PlanDesc> plans;
@@ -472,6 +473,7 @@ int nsg_tran_batch_run(nsg_tran_batch* b, void* stream) {
                 break;
             }
             if (b->topos.size() != ntopos) {  // new plans to upload
+                build_programs(b->topos, ntopos);
                 int rc = refresh_plans(b->topos, &b->d_lu_pool, &b->d_plans, &b->max_col,
                                        &b->max_n);
                 if (rc != NSG_OK) return rc;
