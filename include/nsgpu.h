@@ -543,9 +543,9 @@ int nsg_tran_batch_create(int count, nsg_circuit* const* circuits, double tstep,
 void nsg_tran_batch_free(nsg_tran_batch* b);
 /* Launch shape of the transient kernel: threads per CTA (128, 256 or 512)
  * and CTAs per SM (128: 8; 256: 4; 512: 2; 0 = that default), or 0, 0 for
- * the automatic choice (512 for a few hundred instances or any instance
- * above 128 unknowns; else 128 or 256, enough for one pass of the device
- * loads).  Tuning only: the shapes give the same results.  No counterpart
+ * the automatic choice (512 for any instance above 128 unknowns; else 128
+ * or 256, enough for one pass of the device loads, four or two CTAs per
+ * SM, one for up to one instance per SM).  Tuning only: the shapes give the same results.  No counterpart
  * in the reference. */
 int nsg_tran_batch_set_shape(nsg_tran_batch* b, int threads, int blocks_per_sm);
 /* Run the whole batch on a stream.  Instances stop for the host when a
