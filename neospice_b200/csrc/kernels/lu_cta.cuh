@@ -293,7 +293,8 @@ __device__ __forceinline__ void run_step(bool amd, const double* lu, double* buf
 // warp's row -> position scratch (pd.n words), written for column j's rows
 // first.  The row map reads L(:, r)'s row indices, which every consumer
 // column of r shares, instead of a map entry per update.
-template <bool kCrossSm, int kPlan, int kDest, int kChunk = kColChunk, class Probe, class Publish>
+template <bool kCrossSm, int kPlan, int kDest, int kChunk = kColChunk, int kGroupN = kGroup,
+          class Probe, class Publish>
 __device__ __forceinline__ void refactor_column(
     const PlanDesc& pd, const int32_t* __restrict__ pool, const double* __restrict__ a,
     double* lu, double diag_gmin, int check_pivots, double rel_threshold, int32_t j, double* buf,
@@ -307,6 +308,7 @@ __device__ __forceinline__ void refactor_column(
     const bool amd = kPlan < 0 ? pd.kind == kPlanAmdLu : kPlan == kPlanAmdLu;
     const int32_t* piv_rank = pool + pd.off[PA_piv_rank];
     const int32_t* gmin_pos = pool + pd.off[PA_gmin_pos];
+    constexpr int kLanes = kGroupN > kRunLanes ? kGroupN : kRunLanes;
     const int lane = threadIdx.x & 31;
 
     const int32_t c0 = col_ptr[j];
@@ -344,11 +346,11 @@ __device__ __forceinline__ void refactor_column(
     };
     window(0);
     for (int32_t q = 0; q < dj;) {
-        if (q - base > 32 - kRunLanes && base + 32 < dj) window(q);
+        if (q - base > 32 - kLanes && base + 32 < dj) window(q);
         const int32_t k0 = q - base;
         // How many of the next entries' source columns are done, at least one.
-        const int32_t ahead = min(min(kRunLanes, dj - q), 32 - k0);
-        const int32_t src = __shfl_sync(0xffffffffu, meta.x, k0 + (lane & (kRunLanes - 1)));
+        const int32_t ahead = min(min(kLanes, dj - q), 32 - k0);
+        const int32_t src = __shfl_sync(0xffffffffu, meta.x, k0 + (lane & (kLanes - 1)));
         int32_t ready = 0;
         for (int spins = 0;;) {
             const bool open = lane < ahead && probe(src) == 0;
@@ -377,11 +379,11 @@ __device__ __forceinline__ void refactor_column(
             // Up to kGroup entries of any structure: the first 32 rows of
             // every L(:, r), their destinations and the pivot reciprocals
             // are loaded together, then applied one entry after another.
-            const int32_t count = min(kGroup, ready);
-            int32_t l0[kGroup], cnt[kGroup], us[kGroup], dd[kGroup];
-            double rd[kGroup], ll[kGroup];
+            const int32_t count = min(kGroupN, ready);
+            int32_t l0[kGroupN], cnt[kGroupN], us[kGroupN], dd[kGroupN];
+            double rd[kGroupN], ll[kGroupN];
 #pragma unroll
-            for (int g = 0; g < kGroup; ++g) {
+            for (int g = 0; g < kGroupN; ++g) {
                 const int32_t k = k0 + min(g, count - 1);
                 const int32_t dp = __shfl_sync(0xffffffffu, meta.y, k);
                 l0[g] = dp + 1;
@@ -393,7 +395,7 @@ __device__ __forceinline__ void refactor_column(
                 dd[g] = lane < cnt[g] ? dest(us[g], l0[g], lane) : 0;
             }
 #pragma unroll
-            for (int g = 0; g < kGroup; ++g) {
+            for (int g = 0; g < kGroupN; ++g) {
                 if (g < count) {
                     const double u = amd ? buf[q + g] : lu_mul(buf[q + g], rd[g]);
                     colmax = fmax(colmax, fabs(u));

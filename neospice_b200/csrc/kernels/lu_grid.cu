@@ -27,8 +27,12 @@ namespace {
 constexpr int kGridWarps = 8;    // warps per CTA of the grid-wide sweeps
 // Rounds of 32 rows of L(:, r) a warp loads before applying them: long L
 // columns (the separators' hundreds of rows) then cost one L2 round trip
-// per 512 rows instead of per 128.
-constexpr int kGridChunk = 16;
+// per 256 rows instead of per 128.
+constexpr int kGridChunk = 8;
+// U entries whose operands a warp loads together (with 16 rounds and two entries
+// a 16,393-unknown power grid's refactor took 5.05 ms, with 8 and four 4.74 ms,
+// with eight entries 5.2 ms or more).
+constexpr int kGridGroup = 4;
 constexpr int kGridThreads = kGridWarps * 32;
 // CTAs per SM of the grid-wide sweeps.
 constexpr int kGridSolveBlocks = 2;
@@ -317,7 +321,7 @@ grid_refactor_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restri
         const int32_t len = col_ptr[j + 1] - col_ptr[j];
         double* buf = (len <= kColbuf) ? sbuf : lu + col_ptr[j];
         auto probe = [&](int32_t r) { return gflag_acquire(done + r); };
-        refactor_column<true, -1, -1, kGridChunk>(
+        refactor_column<true, -1, -1, kGridChunk, kGridGroup>(
             pd, pool, A + id.a_off, lu, diag_gmin, check_pivots, rel_threshold, j, buf, lr, ur,
             probe,
             [&](const ColumnResult& c) {
