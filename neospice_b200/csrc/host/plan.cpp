@@ -366,7 +366,7 @@ void finish(TopologyPlan& p) {
 }  // namespace
 
 // The level program of a Markowitz plan (see TopologyPlan::lp), for factors
-// within the bounds above.  An entry of the factor receives its updates in
+// within the bounds above that have an update map.  An entry of the factor receives its updates in
 // ascending pivot order, a row of a sweep its columns in the order of the
 // row-wise sweeps, so every value is the one the column-wise refactor and the
 // sweeps compute.
@@ -376,7 +376,7 @@ void build_level_program(TopologyPlan& p) {
     const int32_t n = p.n, nlu = p.nnz_lu;
     const int32_t vec = nlu, pivots = nlu + n, zero = nlu + 2 * n, one = zero + 1;
     static_assert(8 * kLevelMaxDoubles <= 0xffff, "value offsets are 16 bits");
-    if (p.kind != kPlanKindMarkowitz || one >= kLevelMaxDoubles ||
+    if (p.kind != kPlanKindMarkowitz || !p.has_update_map || one >= kLevelMaxDoubles ||
         p.updates > kLevelMaxUpdatesPerRow * n || p.nnz_a >= 0xffff)
         return;
     // updates of each LU position, ascending in the source column

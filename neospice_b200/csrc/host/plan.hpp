@@ -190,7 +190,7 @@ TopologyPlan build_plan(const MarkowitzOrder& mo, const std::vector<int32_t>& sl
 TopologyPlan build_plan_amd(const AmdLuFactor& f);
 
 // Give a plan its level program (TopologyPlan::lp) if it is a small sparse
-// Markowitz plan; clears it otherwise.  The batches of circuits call it for
+// Markowitz plan with an update map; clears it otherwise.  The batches of circuits call it for
 // each distinct plan they keep.
 void build_level_program(TopologyPlan& p);
 
