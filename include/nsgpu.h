@@ -38,8 +38,11 @@ typedef struct nsg_batch nsg_batch;
 const char* nsg_last_error(void);
 
 /* Polls a dependency wait inside the dataflow and grid-wide kernels makes
- * before it gives up; the instance then reports NSG_TIMEOUT (104) and the
- * kernel still runs to its end, so the context stays usable.  Default 2^22
+ * before it gives up.  A refactor, Newton or adjoint kernel then reports
+ * NSG_TIMEOUT (104) for the instance; the kernel still runs to its end, so the
+ * context stays usable.  The batched solves (real, transposed, complex and
+ * grid-wide) start over level after level, without waits, and give the same
+ * values as ever.  Default 2^22
  * polls (seconds; a wait that runs out means a broken schedule, not a slow
  * one).  0 gives up at the first wait that has to poll -- used by tests to
  * exercise the give-up path.  Applies to every kernel of the library on the

@@ -228,9 +228,10 @@ complex_flow_refactor_kernel(const PlanDesc* __restrict__ plans, const int32_t* 
 // 32 entries and flags at once, products in parallel, subtractions in order.
 // kForward: L, entries with a zero operand left out, then the reciprocal pivot
 // unless the row is zero; else U.  The factor is read through the plan's row
-// positions (pos), the vector and the flags are in shared memory.
+// positions (pos), the vector and the flags are in shared memory.  False if a
+// bounded wait gave up.
 template <bool kForward>
-__device__ __forceinline__ void c_sweep_rows(const int32_t* order, const int32_t* ptr,
+__device__ __forceinline__ bool c_sweep_rows(const int32_t* order, const int32_t* ptr,
                                              const int32_t* idx, const int32_t* pos,
                                              const int32_t* diag_pos, const double2* lu, int32_t n,
                                              double2* w, volatile int32_t* done, int32_t target) {
@@ -315,11 +316,17 @@ __device__ __forceinline__ void c_sweep_rows(const int32_t* order, const int32_t
             v = nv;
         }
     }
+    return ok;
 }
+
+// Level after level, a thread per row (below).
+__device__ void c_solve_levels(const PlanDesc& pd, const int32_t* pool, const double* lu, double* x,
+                               double* w);
 
 // x <- A^{-1} x for one instance per CTA with dataflow sweeps.  Level after
 // level with a thread per row and the vector in global memory, 150 points of a
-// 1026-unknown mesh took 1.81 ms, here 0.35 ms.
+// 1026-unknown mesh took 1.81 ms, here 0.35 ms.  If a bounded wait gave up,
+// x still holds the right-hand side and is solved level after level.
 template <int kThreads, int kBlocks>
 __global__ void __launch_bounds__(kThreads, kBlocks)
 complex_flow_solve_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restrict__ pool,
@@ -335,19 +342,26 @@ complex_flow_solve_kernel(const PlanDesc* __restrict__ plans, const int32_t* __r
     const double2* lu = reinterpret_cast<const double2*>(LU) + id.lu_off;
     double* x = X + 2 * id.x_off;
     volatile int32_t* done = reinterpret_cast<volatile int32_t*>(cols + n);
+    __shared__ int32_t s_ok;
+    if (threadIdx.x == 0) s_ok = 1;
     for (int32_t i = threadIdx.x; i < n; i += blockDim.x) {
         cols[i] = make_double2(x[2 * perm_row[i]], x[2 * perm_row[i] + 1]);
         done[i] = 0;
     }
     __syncthreads();
-    c_sweep_rows<true>(pool + pd.off[PA_fwd_lev], pool + pd.off[PA_lrow_ptr],
-                       pool + pd.off[PA_lrow_col], pool + pd.off[PA_lrow_pos], diag_pos, lu, n, cols,
-                       done, 1);
+    bool ok = c_sweep_rows<true>(pool + pd.off[PA_fwd_lev], pool + pd.off[PA_lrow_ptr],
+                                 pool + pd.off[PA_lrow_col], pool + pd.off[PA_lrow_pos], diag_pos,
+                                 lu, n, cols, done, 1);
     __syncthreads();
-    c_sweep_rows<false>(pool + pd.off[PA_bwd_lev], pool + pd.off[PA_urow_ptr],
-                        pool + pd.off[PA_urow_col], pool + pd.off[PA_urow_pos], diag_pos, lu, n,
-                        cols, done, 2);
+    ok = c_sweep_rows<false>(pool + pd.off[PA_bwd_lev], pool + pd.off[PA_urow_ptr],
+                             pool + pd.off[PA_urow_col], pool + pd.off[PA_urow_pos], diag_pos, lu,
+                             n, cols, done, 2) && ok;
+    if (!ok) s_ok = 0;
     __syncthreads();
+    if (s_ok == 0) {
+        c_solve_levels(pd, pool, LU + 2 * id.lu_off, x, reinterpret_cast<double*>(cols));
+        return;
+    }
     for (int32_t i = threadIdx.x; i < n; i += blockDim.x) {
         x[2 * perm_col[i]] = cols[i].x;
         x[2 * perm_col[i] + 1] = cols[i].y;
@@ -460,24 +474,16 @@ complex_refactor_kernel(const PlanDesc* __restrict__ plans, const int32_t* __res
                                      : (s_fail != 0x7fffffff ? kStatusSingular : kStatusOk);
 }
 
-// The general solve (as the general refactor).
-// x <- A^{-1} x for one instance per CTA, level-synchronous: rows of a level
-// in parallel, each accumulating its updates in the reference's order
-// (forward: columns ascending, skipping zero x_c; backward: row dot in
-// ascending column order).  w: 2n doubles of scratch.
-__global__ void __launch_bounds__(kCplxThreads)
-complex_solve_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restrict__ pool,
-                     const InstDesc* __restrict__ insts, const double* __restrict__ LU,
-                     double* X, double* W) {
-    const InstDesc id = insts[blockIdx.x];
-    const PlanDesc& pd = plans[id.plan];
+// x <- A^{-1} x by the whole CTA, level-synchronous: rows of a level in parallel,
+// each accumulating its updates in the reference's order (forward: columns
+// ascending, skipping zero x_c; backward: row dot in ascending column order).
+// w: 2n doubles of scratch.
+__device__ __noinline__ void c_solve_levels(const PlanDesc& pd, const int32_t* pool,
+                                            const double* lu, double* x, double* w) {
     const int32_t n = pd.n;
     const int32_t* perm_row = pool + pd.off[PA_perm_row];
     const int32_t* perm_col = pool + pd.off[PA_perm_col];
     const int32_t* diag_pos = pool + pd.off[PA_diag_pos];
-    const double* lu = LU + 2 * id.lu_off;
-    double* x = X + 2 * id.x_off;
-    double* w = W + 2 * id.w_off;
     for (int32_t i = threadIdx.x; i < n; i += blockDim.x) {
         w[2 * i] = x[2 * perm_row[i]];
         w[2 * i + 1] = x[2 * perm_row[i] + 1];
@@ -541,6 +547,15 @@ complex_solve_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restri
         x[2 * perm_col[i]] = w[2 * i];
         x[2 * perm_col[i] + 1] = w[2 * i + 1];
     }
+}
+
+// The general solve (as the general refactor), one instance per CTA.
+__global__ void __launch_bounds__(kCplxThreads)
+complex_solve_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restrict__ pool,
+                     const InstDesc* __restrict__ insts, const double* __restrict__ LU,
+                     double* X, double* W) {
+    const InstDesc id = insts[blockIdx.x];
+    c_solve_levels(plans[id.plan], pool, LU + 2 * id.lu_off, X + 2 * id.x_off, W + 2 * id.w_off);
 }
 
 }  // namespace

@@ -635,6 +635,16 @@ __device__ inline void cta_solve(const PlanDesc& pd, const int32_t* __restrict__
     __syncthreads();
 }
 
+// cta_solve out of line, for kernels that reach it only where a bounded wait of
+// their dataflow sweeps gave up.
+static __device__ __noinline__ void cta_solve_levels(const PlanDesc& pd,
+                                                     const int32_t* __restrict__ pool,
+                                                     const double* __restrict__ lu,
+                                                     double* __restrict__ x,
+                                                     double* __restrict__ w) {
+    cta_solve(pd, pool, lu, x, w);
+}
+
 // Dynamic shared memory of a Newton kernel launch: the LU scratch (flow or
 // small path) followed by an optional stage for instance workspaces, capped
 // so that two CTAs still fit on an SM.
@@ -1131,8 +1141,8 @@ struct SweepRows {
 // unknown mesh where this takes 0.48 ms (B200, 1965 MHz).
 // Rows are dealt to warps in level order, and a row waits only on rows at
 // earlier positions, so every wait ends; waits are bounded all the same
-// (c_wait_limit polls without progress, then the row runs on with what it has
-// and the sweep reports false).
+// (c_wait_limit polls in vain within 32 entries, then the warp runs on with
+// what it has and the sweep reports false).
 template <int kFinal, bool kSkipZero, bool kDescending>
 __device__ __forceinline__ bool sweep_rows(const SweepRows& s, int32_t n, double* w,
                                            volatile int32_t* done, int32_t target) {
@@ -1223,8 +1233,9 @@ __device__ __forceinline__ bool sweep_rows(const SweepRows& s, int32_t n, double
 
 // The two sweeps of a dataflow solve with the vector and its flags in shared
 // memory (flow_solve_smem_bytes): gather through perm_in, first sweep (flags
-// to 1), second sweep (flags to 2), scatter through perm_out.  Returns false
-// if a bounded wait gave up.  Begins and ends with __syncthreads().
+// to 1), second sweep (flags to 2), scatter through perm_out.  Returns false,
+// with x as it was, if a bounded wait gave up.  Begins and ends with
+// __syncthreads().
 template <class First, class Second>
 __device__ __forceinline__ bool sweep_pair(int32_t n, const int32_t* perm_in,
                                            const int32_t* perm_out, double* __restrict__ x,
@@ -1244,8 +1255,9 @@ __device__ __forceinline__ bool sweep_pair(int32_t n, const int32_t* perm_in,
     ok = second(w, done) && ok;
     if (!ok) s_ok = 0;
     __syncthreads();
-    for (int32_t i = threadIdx.x; i < n; i += blockDim.x) x[perm_out[i]] = w[i];
     const bool all_ok = (s_ok != 0);
+    if (all_ok)
+        for (int32_t i = threadIdx.x; i < n; i += blockDim.x) x[perm_out[i]] = w[i];
     __syncthreads();
     return all_ok;
 }
@@ -1285,8 +1297,15 @@ static __device__ __noinline__ bool cta_solve_flow(const PlanDesc& pd, const int
 // reciprocal pivot (AMD-LU: A^T = Q U^T L^T P, U^T with the pivot division, then
 // unit L^T).  Same arithmetic, in the same order per row, as
 // cta_solve_transposed: 592 transposed solves of 145 to 577 unknowns took
-// 0.67 ms with a thread per row and a barrier per level, 0.36 ms here.
-static __device__ __noinline__ bool cta_solve_transposed_flow(const PlanDesc& pd,
+// 0.67 ms with a thread per row and a barrier per level, 0.36 ms here.  If a
+// bounded wait gave up, those sweeps, which wait for nothing but barriers, give
+// the result (the vector in smem).
+static __device__ __noinline__ void cta_solve_transposed_levels(const PlanDesc& pd,
+                                                                const int32_t* __restrict__ pool,
+                                                                const double* __restrict__ lu,
+                                                                double* __restrict__ x,
+                                                                double* __restrict__ w);
+static __device__ __noinline__ void cta_solve_transposed_flow(const PlanDesc& pd,
                                                               const int32_t* __restrict__ pool,
                                                               const double* __restrict__ lu,
                                                               double* __restrict__ x,
@@ -1298,7 +1317,7 @@ static __device__ __noinline__ bool cta_solve_transposed_flow(const PlanDesc& pd
     const int32_t* row_idx = pool + pd.off[PA_row_idx];
     const SweepRows over_u{pool + pd.off[PA_col_lev], cp, diag_pos, 0, row_idx, lu, diag_pos, lu};
     const SweepRows over_l{pool + pd.off[PA_tbw_lev], diag_pos, cp + 1, 1, row_idx, lu, diag_pos, lu};
-    return sweep_pair(
+    const bool ok = sweep_pair(
         n, pool + pd.off[PA_perm_col], pool + pd.off[PA_perm_row], x, smem,
         [&](double* w, volatile int32_t* done) {
             return amd ? sweep_rows<kFinalDiv, true, false>(over_u, n, w, done, 1)
@@ -1308,10 +1327,12 @@ static __device__ __noinline__ bool cta_solve_transposed_flow(const PlanDesc& pd
             return amd ? sweep_rows<kFinalNone, false, false>(over_l, n, w, done, 2)
                        : sweep_rows<kFinalMul, false, false>(over_l, n, w, done, 2);
         });
+    if (!ok) cta_solve_transposed_levels(pd, pool, lu, x, smem);
 }
 
-// The same level after level, a thread per row, with the vector in global
-// memory: for instances whose vector and flags exceed shared memory.
+// The same level after level, a thread per row; w is an n-vector of scratch: for
+// instances whose vector and flags exceed shared memory, and where a wait gave
+// up.
 // x <- A^{-T} x (SparseMatrix::solve_transposed) by the whole CTA.  AMD-LU
 // plans (the reference's AmdLuSolver has no transposed solve) use
 // A^T = Q U^T L^T P: U^T forward with the pivot division, then unit L^T.
@@ -1361,6 +1382,14 @@ __device__ inline void cta_solve_transposed(const PlanDesc& pd, const int32_t* _
     }
     for (int32_t i = threadIdx.x; i < n; i += blockDim.x) x[perm_row[i]] = w[i];
     __syncthreads();
+}
+
+static __device__ __noinline__ void cta_solve_transposed_levels(const PlanDesc& pd,
+                                                                const int32_t* __restrict__ pool,
+                                                                const double* __restrict__ lu,
+                                                                double* __restrict__ x,
+                                                                double* __restrict__ w) {
+    cta_solve_transposed(pd, pool, lu, x, w);
 }
 
 }  // namespace nsg

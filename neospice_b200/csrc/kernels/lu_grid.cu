@@ -534,13 +534,19 @@ grid_solve_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restrict_
     if (!ok) atomicExch(&st->timeout, 1);
 }
 
-// x through perm_col from the backward sweep's rows.
+// x through perm_col from the backward sweep's rows.  If a bounded wait gave up,
+// x still holds the right-hand side, and one CTA solves level after level.
 __global__ void __launch_bounds__(kGridThreads)
 grid_scatter_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restrict__ pool,
-                    const InstDesc* __restrict__ insts, int inst, const double* __restrict__ wb,
+                    const InstDesc* __restrict__ insts, int inst, const double* __restrict__ LU,
+                    double* __restrict__ wb, const GridState* __restrict__ st,
                     double* __restrict__ X) {
     const InstDesc id = insts[inst];
     const PlanDesc& pd = plans[id.plan];
+    if (st->timeout) {
+        if (blockIdx.x == 0) cta_solve_levels(pd, pool, LU + id.lu_off, X + id.x_off, wb);
+        return;
+    }
     const int32_t* perm_col = pool + pd.off[PA_perm_col];
     const int32_t i = blockIdx.x * kGridThreads + threadIdx.x;
     if (i < pd.n) X[id.x_off + perm_col[i]] = wb[i];
@@ -666,9 +672,7 @@ cudaError_t launch_grid_refactor(const PlanDesc* plans, const int32_t* pool,
 }
 
 // x <- A^{-1} x for every instance in turn with the whole GPU (needs the
-// row-major copies written by a dataflow or grid-wide refactor).  A bounded
-// wait that gave up leaves that instance's result undefined, as in the
-// batched sweeps.
+// row-major copies written by a dataflow or grid-wide refactor).
 cudaError_t launch_grid_solve(const PlanDesc* plans, const int32_t* pool, const InstDesc* insts,
                               int count, const int32_t* n_of, int max_n, const double* LU,
                               const double* lrows, const double* urows, double* X, void* scratch,
@@ -685,7 +689,7 @@ cudaError_t launch_grid_solve(const PlanDesc* plans, const int32_t* pool, const 
         grid_solve_kernel<<<blocks, kGridThreads, 0, stream>>>(plans, pool, insts, i, LU, lrows,
                                                                urows, X, wf, wb, st);
         grid_scatter_kernel<<<(n_of[i] + kGridThreads - 1) / kGridThreads, kGridThreads, 0, stream>>>(
-            plans, pool, insts, i, wb, X);
+            plans, pool, insts, i, LU, wb, st, X);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     return cudaSuccess;

@@ -174,7 +174,8 @@ solve_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restrict__ poo
     cta_solve(plans[inst.plan], pool, LU + inst.lu_off, X + inst.x_off, W + inst.w_off);
 }
 
-// x <- A^{-1} x, dataflow sweeps on the row-major copies (cta_solve_flow).
+// x <- A^{-1} x, dataflow sweeps on the row-major copies (cta_solve_flow), or level
+// after level if one of their bounded waits gave up.
 template <int kThreads, int kBlocks>
 __global__ void __launch_bounds__(kThreads, kBlocks)
 solve_flow_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restrict__ pool,
@@ -183,8 +184,9 @@ solve_flow_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restrict_
                   double* __restrict__ X) {
     extern __shared__ double smem[];
     const InstDesc inst = insts[blockIdx.x];
-    cta_solve_flow(plans[inst.plan], pool, LU + inst.lu_off, lrows + inst.lrows_off,
-                   urows + inst.urows_off, X + inst.x_off, smem);
+    if (!cta_solve_flow(plans[inst.plan], pool, LU + inst.lu_off, lrows + inst.lrows_off,
+                        urows + inst.urows_off, X + inst.x_off, smem))
+        cta_solve_levels(plans[inst.plan], pool, LU + inst.lu_off, X + inst.x_off, smem);
 }
 
 // x <- A^{-T} x with the same LU (SparseMatrix::solve_transposed).

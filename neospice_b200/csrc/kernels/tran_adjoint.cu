@@ -430,11 +430,9 @@ tran_adjoint_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restric
         return cta_refactor_flow(pd, pool, v.a, v.lu, opt.diag_gmin, kCheckNone, 1e-3, smem,
                                  colbuf, v.lrows, v.urows);
     };
-    auto solve_transposed = [&]() -> bool {
-        if (!level_ready(pd, scratch_doubles))
-            return cta_solve_transposed_flow(pd, pool, v.lu, lam, smem);
-        cta_level_solve_transposed(pd, lam);
-        return true;
+    auto solve_transposed = [&] {
+        if (level_ready(pd, scratch_doubles)) cta_level_solve_transposed(pd, lam);
+        else cta_solve_transposed_flow(pd, pool, v.lu, lam, smem);
     };
 
     // ---- 1. operating point: re-solved with the replayed parameters by
@@ -603,10 +601,7 @@ tran_adjoint_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restric
             if (v.n_mos > 0)
                 mos_charge_rhs(v, mos_base, xs, x1, cf, eta1, eta2, mu, kap1, cap1, w1, p1, lam);
             __syncthreads();
-            if (!solve_transposed()) {
-                fail_with(kStatusTimeout);
-                return;
-            }
+            solve_transposed();
             // capacitor adjoints and dL/dC
             for (int32_t k = threadIdx.x; k < v.n_caps; k += blockDim.x) {
                 const int32_t* cr = v.caps + 5 * k;
@@ -691,10 +686,7 @@ tran_adjoint_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restric
     if (v.n_mos > 0)
         mos_charge_rhs(v, mos_base, x0, x0, cf0, eta1, eta2, mu, kap1, cap1, w1, p1, lam);
     __syncthreads();
-    if (!solve_transposed()) {
-        fail_with(kStatusTimeout);
-        return;
-    }
+    solve_transposed();
     if (v.n_mos > 0) {
         mos_charge_update(v, mos_base, x0, x0, cf0, lam, eta1, eta2, mu, kap1, cap1, w1, p1,
                           g);
