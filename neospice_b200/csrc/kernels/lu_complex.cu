@@ -573,7 +573,7 @@ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 
 template <class Kernel, class... Args>
 cudaError_t launch_complex(Kernel kernel, int count, int threads, size_t smem, cudaStream_t stream,
                            Args... args) {
-    if (smem > 48 * 1024) {  // more than a launch may use unasked
+    if (smem > kUnaskedSmem) {
         const cudaError_t e = cudaFuncSetAttribute(
             kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kMaxCplxSmem));
         if (e != cudaSuccess) return e;
@@ -611,7 +611,7 @@ cudaError_t launch_complex_refactor(const PlanDesc* plans, const int32_t* pool,
                               wide, stream, plans, pool, insts, A, LU, status, colbuf);
     }
     const size_t smem = complex_refactor_smem(max_n);
-    if (smem > 48 * 1024) {
+    if (smem > kUnaskedSmem) {
         const cudaError_t e = cudaFuncSetAttribute(
             complex_refactor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         if (e != cudaSuccess) return e;

@@ -196,6 +196,10 @@ __device__ __forceinline__ unsigned long long fail_key(int32_t step, int32_t cod
            static_cast<uint32_t>(code);
 }
 
+// Dynamic shared memory a kernel may use without asking: 48 KB less its static
+// shared memory, for which 1 KB is left.
+constexpr size_t kUnaskedSmem = 47 * 1024;
+
 // Shared memory of the dataflow refactor: a column buffer of colbuf doubles per
 // warp, then n int32 completion flags.
 __host__ __device__ inline size_t flow_smem_bytes(int colbuf, int n, int warps = kFlowWarps) {

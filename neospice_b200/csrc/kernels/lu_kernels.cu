@@ -234,7 +234,7 @@ constexpr int kMaxFlowSmem = 200 * 1024;
 template <class Kernel, class... Args>
 cudaError_t launch_flow(Kernel kernel, int count, int threads, size_t smem, cudaStream_t stream,
                         Args... args) {
-    if (smem > 48 * 1024) {  // more than a launch may use unasked
+    if (smem > kUnaskedSmem) {
         const cudaError_t e =
             cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxFlowSmem);
         if (e != cudaSuccess) return e;
