@@ -297,11 +297,8 @@ std::vector<int64_t> stage_lens(const std::vector<nsg::DcDesc>& ds) {
 }
 
 PlanStage plan_stage(const std::vector<std::unique_ptr<nsg_topology>>& topos, bool transposed) {
-    PlanStage s{0, 0};
-    for (const auto& t : topos) {
-        s.doubles = std::max(s.doubles, t->plan.lp_doubles());
-        s.words = std::max(s.words, t->plan.stage_words(transposed));
-    }
+    PlanStage s;
+    for (const auto& t : topos) s.add(t->plan, transposed);
     return s;
 }
 

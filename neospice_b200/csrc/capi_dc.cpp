@@ -19,7 +19,7 @@ cudaError_t launch_newton_dc(const PlanDesc* plans, const int32_t* lu_pool, cons
                              const double* params, double* work, double* solutions,
                              int32_t* status, int32_t* iterations, DcCtl* ctls,
                              const NewtonOptions& opt, int max_col, int max_n,
-                             const int64_t* stage_lens, int n_stage, int lp_doubles,
+                             const int64_t* stage_lens, int n_stage, int lu_doubles,
                              int plan_words, int32_t* rmaps, cudaStream_t stream);
 size_t dc_smem_bytes(int max_col, int max_n);
 cudaError_t launch_dc_adjoint(const PlanDesc* plans, const int32_t* lu_pool, const DcDesc* descs,

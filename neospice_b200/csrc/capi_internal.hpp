@@ -139,11 +139,8 @@ void place_dcsave(nsg::DcDesc& d, int64_t& work);
 // The instances' stage_len (doubles), ascending.
 std::vector<int64_t> stage_lens(const std::vector<nsg::DcDesc>& ds);
 
-// Shared memory the plans of a batch ask of a Newton kernel: the largest
-// level program's working space and the largest staged part of a plan.
-struct PlanStage {
-    int doubles, words;
-};
+// Shared memory the plans of a batch ask of a Newton kernel.
+using nsg::PlanStage;
 PlanStage plan_stage(const std::vector<std::unique_ptr<nsg_topology>>& topos, bool transposed);
 
 // Host (re-)ordering of one instance that stopped on the device.

@@ -34,7 +34,7 @@ cudaError_t launch_tran_adjoint(const PlanDesc* plans, const int32_t* lu_pool, c
                                 const StepRecord* recs, const double* times, const double* rec_x0,
                                 const double* targets, double weight, double* grads, double* loss,
                                 int32_t* status, const NewtonOptions& opt, int max_iter,
-                                int max_col, int max_n, int lp_doubles, int plan_words,
+                                int max_col, int max_n, int lu_doubles, int plan_words,
                                 cudaStream_t stream);
 }  // namespace nsg
 
@@ -123,14 +123,8 @@ namespace {
 
 // Launch shape of a transient batch (nsg::TranShape).
 nsg::TranShape tran_shape(const nsg_tran_batch& b) {
-    nsg::TranShape sh{b.max_col, b.max_n, stage_lens(b.descs), 0, 0, 0, 0, b.force_threads,
-                      b.force_blocks};
-    const PlanStage need = plan_stage(b.topos, false);
-    sh.lp_doubles = need.doubles;
-    sh.plan_words = need.words;
-    for (const auto& t : b.topos)
-        sh.max_small_lu = std::max({sh.max_small_lu, t->plan.nnz_lu + t->plan.n,
-                                    t->plan.lp_doubles()});
+    nsg::TranShape sh{b.max_col, b.max_n, stage_lens(b.descs), plan_stage(b.topos, false), 0,
+                      b.force_threads, b.force_blocks};
     for (const auto& d : b.descs)
         sh.max_devices = std::max({sh.max_devices, d.n_mos, d.n_diodes, d.n_caps, d.n_srcs});
     return sh;

@@ -498,6 +498,14 @@ int32_t TopologyPlan::stage_words(bool transposed) const {
     return n <= 128 && device_words() <= kPlanStageWords ? static_cast<int32_t>(device_words()) : 0;
 }
 
+void PlanStage::add(const TopologyPlan& p, bool transposed) {
+    const bool one_warp = one_warp_factor(p.n, p.nnz_lu);
+    doubles = std::max({doubles, p.lp_doubles(), one_warp ? p.nnz_lu + p.n : 0});
+    words = std::max(words, p.stage_words(transposed));
+    programs = programs || !p.lp.empty();
+    dataflow = dataflow || (p.lp.empty() && !one_warp);
+}
+
 // A packed update map takes one int32 word per two positions.
 int64_t TopologyPlan::device_words() const {
     int64_t w = 0;

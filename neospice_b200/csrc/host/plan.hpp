@@ -42,6 +42,20 @@ class AmdLuFactor;
 
 constexpr int32_t kRunBit = INT32_MIN;  // of TopologyPlan::umeta's third words
 
+// Whether a Newton kernel runs a factor without a level program on one warp in
+// shared memory (cta_refactor_small) rather than on the dataflow kernels: at
+// most 128 unknowns and 512 entries.  A property of the plan alone, so that a
+// circuit runs alike beside any others and in any launch shape.  The line:
+// transients of n fully coupled RC nodes, 400 instances, take 14.6 ms on one
+// warp and 17.4 ms on the dataflow kernels with n = 12, 17.1 and 19.0 with 16,
+// 20.8 and 20.9 with 20 (484 entries), 25.4 and 24.0 with 24 (676), 71 and 37
+// with 40; MOS networks of 60 nodes (936 entries) 430 and 156 ms.  One instance
+// alone is faster on the dataflow kernels from n = 12 on (4.3 and 3.1 ms).
+constexpr int32_t kOneWarpEntries = 512;
+constexpr bool one_warp_factor(int32_t n, int32_t nnz_lu) {
+    return n <= 128 && nnz_lu <= kOneWarpEntries;
+}
+
 // Engines whose pivot sequence a plan replays.
 enum PlanKindHost : int32_t {
     kPlanKindMarkowitz = 0,  // SparseMatrix (Sparse 1.3): U scaled by 1/pivot
@@ -179,6 +193,16 @@ constexpr int32_t kLevelTerms = 2;
 enum LevelFlag : uint32_t {
     kLevelPivot = 1,  // t itself to aux, 1 / t to the target
     kLevelSkip = 2,   // forward sweep: terms with first or first * scale zero are left out
+};
+
+// Shared memory the plans of a batch ask of a Newton kernel: the largest space
+// of a level program or one-warp factor (doubles) and the largest staged part
+// of a plan (words); and whether any plan has a level program, or has none and
+// runs on the dataflow kernels.
+struct PlanStage {
+    int32_t doubles = 0, words = 0;
+    bool programs = false, dataflow = false;
+    void add(const TopologyPlan& p, bool transposed);
 };
 
 // Build from the host ordering engine after order_and_factor.  slot_elem[k]

@@ -665,10 +665,6 @@ inline size_t stage_bytes_for(size_t scratch_bytes, const int64_t* lens, int cou
     return 2 * fit >= count ? sizeof(double) * static_cast<size_t>(lens[fit - 1]) : 0;
 }
 
-__host__ __device__ inline bool small_fits(int n, int nnz_lu, int smem_doubles) {
-    return n <= 128 && nnz_lu + n <= smem_doubles;
-}
-
 // Level programs.  A small sparse factor (an inverter chain, a BSIM4v7 ring, an
 // interconnect tree: a few updates per unknown) is bound by its longest chain
 // of dependent operations, not by their number, and on one warp alone by the

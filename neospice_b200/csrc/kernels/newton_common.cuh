@@ -505,7 +505,7 @@ __device__ inline NewtonOutcome newton(const Inst& v, const PlanDesc& pd, const 
     // warp-level refactor and sweeps, both in shared memory; larger ones use
     // the dataflow schedule over global memory.
     const bool level = level_ready(pd, smem_doubles);
-    const bool small = small_fits(pd.n, pd.nnz_lu, smem_doubles);
+    const bool small = one_warp_factor(pd.n, pd.nnz_lu);
     double* lu_s = smem;
     double* w_s = smem + pd.nnz_lu;
     __syncthreads();

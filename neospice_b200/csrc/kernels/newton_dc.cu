@@ -124,15 +124,15 @@ cudaError_t launch_newton_dc(const PlanDesc* plans, const int32_t* lu_pool, cons
                              const double* params, double* work, double* solutions,
                              int32_t* status, int32_t* iterations, DcCtl* ctls,
                              const NewtonOptions& opt, int max_col, int max_n,
-                             const int64_t* stage_lens, int n_stage, int lp_doubles,
+                             const int64_t* stage_lens, int n_stage, int lu_doubles,
                              int plan_words, int32_t* rmaps, cudaStream_t stream) {
     if (count <= 0) return cudaSuccess;
     const int colbuf = (max_col + 31) & ~31;
     const bool wide = count <= dc_sm_count() &&
                       dc_scratch_bytes(max_col, max_n, kDcMaxWarps) <= 200 * 1024;
-    const size_t level = sizeof(double) * static_cast<size_t>(lp_doubles);
+    const size_t small = sizeof(double) * static_cast<size_t>(lu_doubles);
     const size_t flow = dc_scratch_bytes(max_col, max_n, wide ? kDcMaxWarps : kFlowWarps);
-    const size_t scratch = ((flow > level ? flow : level) + 15) & ~size_t{15};
+    const size_t scratch = ((flow > small ? flow : small) + 15) & ~size_t{15};
     size_t plan = (sizeof(int32_t) * static_cast<size_t>(plan_words) + 15) & ~size_t{15};
     if (scratch + plan > kStageCapBytes) plan = 0;  // read from global memory instead
     const size_t stage = stage_bytes_for(scratch + plan, stage_lens, n_stage);

@@ -704,14 +704,14 @@ cudaError_t launch_tran_adjoint(const PlanDesc* plans, const int32_t* lu_pool, c
                                 const StepRecord* recs, const double* times, const double* rec_x0,
                                 const double* targets, double weight, double* grads, double* loss,
                                 int32_t* status, const NewtonOptions& opt, int max_iter,
-                                int max_col, int max_n, int lp_doubles, int plan_words,
+                                int max_col, int max_n, int lu_doubles, int plan_words,
                                 cudaStream_t stream) {
     if (count <= 0) return cudaSuccess;
     const int colbuf = (max_col + 31) & ~31;
     const size_t a = flow_smem_bytes(colbuf, max_n), b = flow_solve_smem_bytes(max_n);
-    const size_t level = sizeof(double) * static_cast<size_t>(lp_doubles);
+    const size_t small = sizeof(double) * static_cast<size_t>(lu_doubles);
     const size_t flow = a > b ? a : b;
-    const size_t scratch = ((flow > level ? flow : level) + 15) & ~size_t{15};
+    const size_t scratch = ((flow > small ? flow : small) + 15) & ~size_t{15};
     size_t plan = (sizeof(int32_t) * static_cast<size_t>(plan_words) + 15) & ~size_t{15};
     if (scratch + plan > kStageCapBytes) plan = 0;  // read from global memory instead
     const size_t smem = scratch + plan;

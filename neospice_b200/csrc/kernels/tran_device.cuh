@@ -1,6 +1,7 @@
 // Device descriptors of the batched transient kernel.
 #pragma once
 #include "dc_device.cuh"
+#include "host/plan.hpp"
 
 #include <cstdint>
 #include <vector>
@@ -60,16 +61,13 @@ struct TranCtl {
 };
 
 // What the launch needs to size one CTA: the batch's largest LU column and
-// unknown count (dataflow scratch), the instances' staged workspaces, largest
-// shared-memory LU (doubles: nnz_lu + n, or a level program's space), largest
-// space of a level program, most words of a plan to keep in shared memory and
-// most devices of one family in one instance (the device loads' parallelism).
+// unknown count (dataflow scratch), the instances' staged workspaces, what the
+// plans keep in shared memory and most devices of one family in one instance
+// (the device loads' parallelism).
 struct TranShape {
     int32_t max_col, max_n;
     std::vector<int64_t> stage_lens;  // ascending
-    int32_t max_small_lu;
-    int32_t lp_doubles;
-    int32_t plan_words;
+    PlanStage plans;
     int32_t max_devices;
     int32_t force_threads;   // nsg_tran_batch_set_shape (0: automatic)
     int32_t force_blocks;

@@ -507,14 +507,42 @@ transient_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restrict__
     finish(d, work, stage, g, k, o, npoints, status, stats, k.status);
 }
 
-size_t tran_smem_bytes(int max_col, int max_n) {
+namespace {
+
+size_t tran_flow_bytes(int max_col, int max_n, int threads) {
     const int colbuf = (max_col + 31) & ~31;
-    const size_t a = flow_smem_bytes(colbuf, max_n);
+    const size_t a = flow_smem_bytes(colbuf, max_n, threads / 32);
     const size_t b = flow_solve_smem_bytes(max_n);
     return a > b ? a : b;
 }
 
-namespace {
+// Shared memory of a launch shape (bytes, each a multiple of 16): the LU
+// scratch, the staged plan and the staged workspace.
+struct TranSmem {
+    size_t scratch, plan, stage;
+};
+
+TranSmem tran_smem(const TranShape& sh, int threads, int blocks) {
+    const size_t flow = tran_flow_bytes(sh.max_col, sh.max_n, threads);
+    const size_t small = sizeof(double) * static_cast<size_t>(sh.plans.doubles);
+    const size_t words = (sizeof(int32_t) * static_cast<size_t>(sh.plans.words) + 15) & ~size_t{15};
+    TranSmem m;
+    m.scratch = ((flow > small ? flow : small) + 15) & ~size_t{15};
+    // The CTA's share of the SM's 228 KB, less its static shared memory and the
+    // 1 KB the runtime reserves per CTA; the rest of a larger share is better
+    // left to L1.
+    const size_t share = (228 * 1024) / static_cast<size_t>(blocks) - 3 * 1024;
+    const size_t budget = share < kStageCapBytes ? share : kStageCapBytes;
+    m.plan = m.scratch + words <= budget ? words : 0;  // else read from global memory
+    if (threads == kFlowThreads) {
+        m.stage = stage_bytes_for(m.scratch + m.plan, sh.stage_lens.data(),
+                                  static_cast<int>(sh.stage_lens.size()));
+        return m;
+    }
+    const size_t want = sizeof(double) * static_cast<size_t>(sh.stage_lens.back());
+    m.stage = m.scratch + m.plan + want <= budget ? want : 0;
+    return m;
+}
 
 template <int kThreads, int kBlocks>
 cudaError_t configure_transient() {
@@ -539,15 +567,22 @@ int sm_count() {
 
 }  // namespace
 
+size_t tran_smem_bytes(int max_col, int max_n) {
+    return tran_flow_bytes(max_col, max_n, kFlowThreads);
+}
+
 // Launch shapes.  The device loads are long serial chains of one thread each,
 // and at 64 registers a thread they spill; so CTAs are as small as the loads
 // need for one pass, and get as many registers as the instances in flight
-// leave.  When every instance is small (n <= 128):
+// leave.  When every instance is small (n <= 128) and runs its level program or
+// on one warp:
 //   up to one instance per SM   one CTA of 256 threads (255 registers)
 //   more                        CTAs of 128 or 256 threads, as many as the
 //                               largest device family needs (128 registers):
-//                               four or two per SM
-// else CTAs of 512 threads, one per SM (128 registers) or two (64).
+//                               four or two per SM; 256 also where four CTAs
+//                               have no room for the level programs
+// else CTAs of 512 threads, one per SM (128 registers) or two (64): a factor on
+// the dataflow kernels keeps their 16 warps busy.
 // Passes measured on a B200, two CTAs of 512 threads per SM (small batches) or
 // 1024 threads per SM (large ones) -> these: one inverter chain 25.8 -> 20.4
 // ms, 400 chains 37.3 -> 35.4, 1184 chains 94.7 -> 94.3; BSIM4v7 ring + NAND,
@@ -565,43 +600,29 @@ cudaError_t launch_transient(const PlanDesc* plans, const int32_t* lu_pool, cons
     if (count <= 0) return cudaSuccess;
     const int colbuf = (sh.max_col + 31) & ~31;
     const bool alone = count <= sm_count();
+    auto room = [&](int t, int b) {  // for the level programs
+        return !sh.plans.programs || tran_smem(sh, t, b).plan > 0;
+    };
     int threads = kFlowThreads, blocks = alone ? 1 : 2;
-    if (sh.max_n <= 128 && sh.max_devices <= 256) {
-        threads = (alone || sh.max_devices > 128) ? 256 : 128;
-        blocks = alone ? 1 : 512 / threads;
+    if (sh.max_n <= 128 && sh.max_devices <= 256 && !sh.plans.dataflow) {
+        if (!alone && sh.max_devices <= 128 && room(128, 4)) {
+            threads = 128;
+            blocks = 4;
+        } else if (room(256, blocks)) {
+            threads = 256;
+        }
     }
     if (sh.force_threads > 0) {
         threads = sh.force_threads;
         blocks = sh.force_blocks > 0 ? sh.force_blocks : 1024 / threads;
     }
-    const bool small_shape = threads != kFlowThreads;
-    if (small_shape && sh.max_n > 128) return cudaErrorInvalidValue;
-    size_t scratch, plan, stage;
-    if (!small_shape) {
-        const size_t flow = tran_smem_bytes(sh.max_col, sh.max_n);
-        const size_t level = sizeof(double) * static_cast<size_t>(sh.lp_doubles);
-        scratch = ((flow > level ? flow : level) + 15) & ~size_t{15};
-        plan = (sizeof(int32_t) * static_cast<size_t>(sh.plan_words) + 15) & ~size_t{15};
-        if (scratch + plan > kStageCapBytes) plan = 0;  // read from global memory instead
-        stage = stage_bytes_for(scratch + plan, sh.stage_lens.data(),
-                                static_cast<int>(sh.stage_lens.size()));
-    } else {
-        // Per-CTA share of the SM's 228 KB, less the CTA's static shared
-        // memory and the 1 KB the runtime reserves per CTA; the rest of a
-        // larger share is better left to L1.
-        const size_t share = (228 * 1024) / static_cast<size_t>(blocks) - 3 * 1024;
-        const size_t budget = share < kStageCapBytes ? share : kStageCapBytes;
-        scratch = (sizeof(double) * static_cast<size_t>(sh.max_small_lu) + 15) & ~size_t{15};
-        plan = (sizeof(int32_t) * static_cast<size_t>(sh.plan_words) + 15) & ~size_t{15};
-        if (scratch + plan > budget) plan = 0;
-        const size_t want = static_cast<size_t>(sh.stage_lens.back()) * sizeof(double);
-        stage = (scratch + plan + want <= budget) ? want : 0;
-    }
-    const size_t smem = scratch + stage + plan;
+    if (threads != kFlowThreads && sh.max_n > 128) return cudaErrorInvalidValue;
+    const TranSmem m = tran_smem(sh, threads, blocks);
+    const size_t smem = m.scratch + m.stage + m.plan;
     if (smem > 200 * 1024) return cudaErrorInvalidValue;
-    const int scratch_d = static_cast<int>(scratch / sizeof(double));
-    const int stage_d = static_cast<int>(stage / sizeof(double));
-    const int plan_w = static_cast<int>(plan / sizeof(int32_t));
+    const int scratch_d = static_cast<int>(m.scratch / sizeof(double));
+    const int stage_d = static_cast<int>(m.stage / sizeof(double));
+    const int plan_w = static_cast<int>(m.plan / sizeof(int32_t));
     cudaError_t e;
 #define NSG_LAUNCH_TRAN(T, B)                                                                  \
     if ((e = configure_transient<T, B>()) != cudaSuccess) return e;                            \
