@@ -89,14 +89,6 @@ size_t dc_scratch_bytes(int max_col, int max_n, int warps) {
     return a > b ? a : b;
 }
 
-template <int kThreads, int kBlocks>
-cudaError_t configure_dc() {
-    static const cudaError_t e =
-        cudaFuncSetAttribute(newton_dc_kernel<kThreads, kBlocks>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    return e;
-}
-
 int dc_sm_count() {
     static const int sms = [] {
         int dev = 0, n = 0;
@@ -141,17 +133,18 @@ cudaError_t launch_newton_dc(const PlanDesc* plans, const int32_t* lu_pool, cons
     const int scratch_d = static_cast<int>(scratch / sizeof(double));
     const int stage_d = static_cast<int>(stage / sizeof(double));
     const int plan_w = static_cast<int>(plan / sizeof(int32_t));
-    const cudaError_t e = wide ? configure_dc<32 * kDcMaxWarps, 1>() : configure_dc<kFlowThreads, 2>();
-    if (e != cudaSuccess) return e;
-    if (wide)
-        newton_dc_kernel<32 * kDcMaxWarps, 1><<<count, 32 * kDcMaxWarps, smem, stream>>>(
-            plans, lu_pool, descs, subset, prog, params, work, solutions, status, iterations, ctls,
-            opt, colbuf, scratch_d, stage_d, plan_w, rmaps, max_n);
-    else
-        newton_dc_kernel<kFlowThreads, 2><<<count, kFlowThreads, smem, stream>>>(
-            plans, lu_pool, descs, subset, prog, params, work, solutions, status, iterations, ctls,
-            opt, colbuf, scratch_d, stage_d, plan_w, rmaps, max_n);
-    return cudaGetLastError();
+    auto launch = [&](auto kernel, int threads) -> cudaError_t {
+        const cudaError_t e = cudaFuncSetAttribute(
+            kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        if (e != cudaSuccess) return e;
+        kernel<<<count, threads, smem, stream>>>(plans, lu_pool, descs, subset, prog, params, work,
+                                                 solutions, status, iterations, ctls, opt, colbuf,
+                                                 scratch_d, stage_d, plan_w, rmaps, max_n);
+        return cudaGetLastError();
+    };
+    constexpr int kWide = 32 * kDcMaxWarps;
+    return wide ? launch(newton_dc_kernel<kWide, 1>, kWide)
+                : launch(newton_dc_kernel<kFlowThreads, 2>, kFlowThreads);
 }
 
 }  // namespace nsg

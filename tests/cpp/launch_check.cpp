@@ -4,6 +4,7 @@
 //   shapes: transients of circuits with level programs or one-warp factors run
 //     in CTAs of 128 or 256 threads, denser factors on 512 threads, whatever
 //     the batch's size; and a launch has room for every path its plans take.
+//   failures: a runtime call that fails once fails that launch only.
 #include "host/plan.hpp"
 #include "host/sparse_order.hpp"
 #include "kernels/tran_device.cuh"
@@ -46,6 +47,10 @@ cudaError_t launch_transient(const PlanDesc*, const int32_t*, const DcDesc*, con
                              double*, const double*, const int32_t*, double*, double*, int32_t*,
                              int32_t*, int32_t*, TranCtl*, const TranOptions&, const TranShape&,
                              StepRecord*, double*, cudaStream_t);
+cudaError_t launch_newton_dc(const PlanDesc*, const int32_t*, const DcDesc*, const int32_t*, int,
+                             const int32_t*, const double*, double*, double*, int32_t*, int32_t*,
+                             DcCtl*, const NewtonOptions&, int, int, const int64_t*, int, int, int,
+                             int32_t*, cudaStream_t);
 }  // namespace nsg
 
 namespace {
@@ -131,9 +136,26 @@ void transient(const char* what, const std::vector<nsg::TopologyPlan>& plans, in
             expect(smem >= sizeof(double) * (p.nnz_lu + p.n), "one-warp room", p.n, threads);
 }
 
+cudaError_t dc(int count) {
+    const std::vector<int64_t> lens(count, 4096);
+    return nsg::launch_newton_dc(nullptr, nullptr, nullptr, nullptr, count, nullptr, nullptr,
+                                 nullptr, nullptr, nullptr, nullptr, nullptr, nsg::NewtonOptions{},
+                                 100, 500, lens.data(), count, 0, 0, nullptr, nullptr);
+}
+
+void one_failure(int count) {
+    attribute_result = cudaErrorMemoryAllocation;
+    launches = 0;
+    expect(dc(count) == cudaErrorMemoryAllocation && launches == 0, "failing attribute", count);
+    attribute_result = cudaSuccess;
+    expect(dc(count) == cudaSuccess && launches == 1, "launch after a failure", count);
+}
+
 }  // namespace
 
 int main() {
+    one_failure(1);
+    one_failure(600);
     expect(!chain(100).lp.empty() && !mesh(8).lp.empty() && !band(128, 4).lp.empty(), "programs");
     expect(mesh(11).lp.empty() && band(128, 6).lp.empty() && coupled(12).lp.empty(), "no programs");
     for (int count : {1, 148, 149, 296, 297, 1200}) {
