@@ -1,6 +1,7 @@
 // C ABI of libnsgpu (declared in include/nsgpu.h): host symbolic phase, batch
 // set-up and the launches of the batched refactor and sweeps.
 #include "capi_internal.hpp"
+#include "host/threads.hpp"
 #include "kernels/dc_device.cuh"
 
 #include <algorithm>
@@ -245,25 +246,11 @@ int intern_topology(std::vector<std::unique_ptr<nsg_topology>>& topos,
 void build_programs(std::vector<std::unique_ptr<nsg_topology>>& topos, size_t from) {
     const size_t count = topos.size() > from ? topos.size() - from : 0;
     std::atomic<size_t> next{from};
-    std::vector<std::exception_ptr> errs(count);
-    auto work = [&] {
-        for (size_t k; (k = next.fetch_add(1)) < topos.size();) try {
-                nsg::build_level_program(topos[k]->plan);
-            } catch (...) {
-                errs[k - from] = std::current_exception();
-            }
-    };
-    const size_t threads =
-        std::min<size_t>(count / 4, std::max(1u, std::thread::hardware_concurrency()));
-    if (threads <= 1) {
-        work();
-    } else {
-        std::vector<std::thread> pool;
-        for (size_t t = 0; t < threads; ++t) pool.emplace_back(work);
-        for (auto& th : pool) th.join();
-    }
-    for (auto& e : errs)
-        if (e) std::rethrow_exception(e);
+    nsg::on_threads(std::min<size_t>(count / 4, std::max(1u, std::thread::hardware_concurrency())),
+                    [&] {
+                        for (size_t k; (k = next.fetch_add(1)) < topos.size();)
+                            nsg::build_level_program(topos[k]->plan);
+                    });
 }
 
 int reorder_instance(std::vector<std::unique_ptr<nsg_topology>>& topos, int topo,

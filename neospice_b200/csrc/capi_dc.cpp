@@ -2,6 +2,7 @@
 #include "capi_internal.hpp"
 
 #include "host/circuit.hpp"
+#include "host/threads.hpp"
 #include "kernels/mos1_model.cuh"
 #include "kernels/dc_device.cuh"
 
@@ -99,21 +100,10 @@ int64_t align4(int64_t x) { return (x + 3) & ~int64_t{3}; }
 // Run f(i) for i in [0, count) on up to `threads` host threads.
 template <class F>
 void parallel_for(int count, int threads, F&& f) {
-    threads = std::max(1, std::min(threads, count));
     std::atomic<int> next{0};
-    std::vector<std::thread> pool;
-    std::vector<std::exception_ptr> errs(threads);
-    for (int t = 0; t < threads; ++t)
-        pool.emplace_back([&, t] {
-            try {
-                for (int i; (i = next.fetch_add(1)) < count;) f(i);
-            } catch (...) {
-                errs[t] = std::current_exception();
-            }
-        });
-    for (auto& th : pool) th.join();
-    for (auto& e : errs)
-        if (e) std::rethrow_exception(e);
+    nsg::on_threads(std::max(1, std::min(threads, count)), [&] {
+        for (int i; (i = next.fetch_add(1)) < count;) f(i);
+    });
 }
 
 }  // namespace

@@ -2,6 +2,7 @@
 #include "capi_internal.hpp"
 
 #include "host/circuit.hpp"
+#include "host/threads.hpp"
 #include "kernels/mos1_charge_adjoint.cuh"
 #include "kernels/mos1_model.cuh"
 #include "kernels/tran_device.cuh"
@@ -216,19 +217,16 @@ int nsg_tran_batch_create(int count, nsg_circuit* const* circuits, double tstep,
         std::vector<std::unique_ptr<nsg_topology>> ord_dc(count);
         std::vector<int> rc_dc(count, NSG_OK);
         std::atomic<int> next{0};
-        std::vector<std::thread> pool;
-        for (int t = 0; t < std::min(threads, count); ++t)
-            pool.emplace_back([&] {
-                for (int i; (i = next.fetch_add(1)) < count;) {
-                    const auto& c = circuits[i]->c;
-                    std::vector<double> a, r;
-                    c.initjct_values(a, r, o.nopt.gmin);
-                    rc_dc[i] = order_topology(c.num_vars(), c.nnz(), c.col_ptr().data(),
-                                              c.row_idx().data(), a.data(), 0.0, ord_dc[i],
-                                              b->solver[i]);
-                }
-            });
-        for (auto& th : pool) th.join();
+        nsg::on_threads(std::min(threads, count), [&] {
+            for (int i; (i = next.fetch_add(1)) < count;) {
+                const auto& c = circuits[i]->c;
+                std::vector<double> a, r;
+                c.initjct_values(a, r, o.nopt.gmin);
+                rc_dc[i] = order_topology(c.num_vars(), c.nnz(), c.col_ptr().data(),
+                                          c.row_idx().data(), a.data(), 0.0, ord_dc[i],
+                                          b->solver[i]);
+            }
+        });
         for (int i = 0; i < count; ++i)
             if (rc_dc[i] != NSG_OK)
                 return fail(NSG_SINGULAR, "nsg_tran_batch_create: symbolic phase failed for "
@@ -434,15 +432,8 @@ int nsg_tran_batch_run(nsg_tran_batch* b, void* stream) {
                     }
                 }
             };
-            const int nthreads = std::max(1, std::min<int>(nt, static_cast<int>(std::max(
-                                                                 1u, std::thread::hardware_concurrency()))));
-            if (nthreads <= 1) {
-                worker();
-            } else {
-                std::vector<std::thread> pool;
-                for (int t = 0; t < nthreads; ++t) pool.emplace_back(worker);
-                for (auto& th : pool) th.join();
-            }
+            nsg::on_threads(std::min<size_t>(nt, std::max(1u, std::thread::hardware_concurrency())),
+                            worker);
             const size_t ntopos = b->topos.size();
             for (int k = 0; k < nt; ++k) {
                 const int i = todo[k];

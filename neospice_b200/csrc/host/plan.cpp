@@ -2,6 +2,7 @@
 
 #include "amd_lu.hpp"
 #include "sparse_order.hpp"
+#include "threads.hpp"
 
 #include <algorithm>
 #include <atomic>
@@ -246,13 +247,7 @@ void finish(TopologyPlan& p) {
         std::atomic<int32_t> next_col{0};
         const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
         const int nthreads = total >= (int64_t{1} << 25) ? static_cast<int>(std::min(hw, 16u)) : 1;
-        if (nthreads == 1) {
-            fill_columns(next_col, n);
-        } else {
-            std::vector<std::thread> pool;
-            for (int t = 0; t < nthreads; ++t) pool.emplace_back(fill_columns, std::ref(next_col), 64);
-            for (auto& th : pool) th.join();
-        }
+        on_threads(nthreads, [&] { fill_columns(next_col, nthreads == 1 ? n : 64); });
     }
     const int32_t first_bad = std::min(bad_dup.load(), bad_fill.load());
     if (first_bad != INT32_MAX) {
