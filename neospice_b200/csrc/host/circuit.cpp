@@ -631,7 +631,9 @@ void Circuit::initjct_values(std::vector<double>& a, std::vector<double>& rhs, d
     }
     // MOSFETs at MODEDCOP | MODEINITJCT from zero state.
     {
-        std::vector<double> rec(kMosRec, 0.0), st(kB4States, 0.0);
+        // three states of their own: the loads' state pointers do not overlap
+        std::vector<double> rec(kMosRec, 0.0), st(3 * kB4States, 0.0);
+        double *const s0 = st.data(), *const s1 = s0 + kB4States, *const s2 = s1 + kB4States;
         const Mos1Integ ic{0, 0, 0, 0, 0, 0, 1, 0};
         const double v0[4] = {0, 0, 0, 0};
         for (size_t m = 0; m < mos_.size(); ++m) {
@@ -639,11 +641,11 @@ void Circuit::initjct_values(std::vector<double>& a, std::vector<double>& rhs, d
             std::fill(st.begin(), st.end(), 0.0);
             double* t = &tv[mos_term_base() + kMosTerms * m];
             if (mos_[m].family == kFamilyBsim4)
-                bsim4_load(&params_[mos_[m].param], rec.data(), st.data(), st.data(), st.data(),
-                           kM1DcOp | kM1InitJct, ic, gmin, 1e-3, 1e-12, v0, t);
+                bsim4_load(&params_[mos_[m].param], rec.data(), s0, s1, s2, kM1DcOp | kM1InitJct, ic,
+                           gmin, 1e-3, 1e-12, v0, t);
             else
-                mos1_load(&params_[mos_[m].param], rec.data(), st.data(), st.data(), st.data(),
-                          kM1DcOp | kM1InitJct, ic, gmin, v0, t);
+                mos1_load(&params_[mos_[m].param], rec.data(), s0, s1, s2, kM1DcOp | kM1InitJct, ic,
+                          gmin, v0, t);
         }
     }
     // Waveform sources at t = 0.
