@@ -148,7 +148,6 @@ void fill_instance(nsg::DcDesc& d, const nsg::Circuit& c, const nsg::TopologyPla
     d.n_grad = static_cast<int32_t>(c.grad_program().size() / 5);
     d.x_off = work; work = align4(work + d.n);
     d.xold_off = work; work = align4(work + d.n);
-    d.w_off = work; work = align4(work + d.n);
     d.a_off = work; work = align4(work + d.nnz);
     d.lu_off = work; work = align4(work + p.nnz_lu);
     d.lrows_off = work; work = align4(work + p.lrow_ptr[p.n]);

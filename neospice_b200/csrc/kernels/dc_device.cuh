@@ -28,9 +28,9 @@ struct DcDesc {
     int64_t prog_off[DP_COUNT];  // int32-word offsets into the program pool
     int64_t param_off;           // into the caller's parameter array
     int64_t sol_off;             // into the caller's solution array
-    // workspace (doubles): solution, previous iterate, sweep scratch, matrix
-    // values, LU values, term values, diode constants
-    int64_t x_off, xold_off, w_off, a_off, lu_off, tv_off, dconst_off;
+    // workspace (doubles): solution, previous iterate, matrix values, LU
+    // values, term values, diode constants
+    int64_t x_off, xold_off, a_off, lu_off, tv_off, dconst_off;
     int64_t lrows_off, urows_off;  // row-major copies of L and U for the sweeps
     int64_t state_off;             // four state vectors of n_states doubles
     int64_t mrec_off;              // per-MOSFET persistent load values
