@@ -3,6 +3,7 @@
 #include "capi_internal.hpp"
 #include "host/threads.hpp"
 #include "kernels/dc_device.cuh"
+#include "kernels/flow_shape.cuh"
 
 #include <algorithm>
 #include <atomic>
@@ -19,13 +20,13 @@
 
 namespace nsg {
 cudaError_t launch_refactor(const PlanDesc* plans, const int32_t* pool, const InstDesc* insts,
-                            int count, const double* A, double* LU, double diag_gmin,
+                            const FlowBatch& b, const double* A, double* LU, double diag_gmin,
                             int check_pivots, double rel_threshold, int32_t* status,
-                            int32_t* fail_step, int max_col, int max_n, bool allow_flow,
-                            double* lrows, double* urows, cudaStream_t stream);
+                            int32_t* fail_step, bool allow_flow, double* lrows, double* urows,
+                            cudaStream_t stream);
 cudaError_t launch_solve(const PlanDesc* plans, const int32_t* pool, const InstDesc* insts,
-                         int count, const double* LU, double* X, double* W, bool transposed,
-                         const double* lrows, const double* urows, int max_n,
+                         const FlowBatch& b, const double* LU, double* X, double* W,
+                         bool transposed, const double* lrows, const double* urows,
                          cudaStream_t stream);
 size_t grid_scratch_bytes(int max_n);
 cudaError_t launch_grid_refactor(const PlanDesc* plans, const int32_t* pool,
@@ -37,12 +38,11 @@ cudaError_t launch_grid_refactor(const PlanDesc* plans, const int32_t* pool,
                                  const int32_t* cta_from_of, cudaStream_t stream);
 int64_t grid_rmap_words(int colbuf, int max_col, int max_n);
 cudaError_t launch_complex_refactor(const PlanDesc* plans, const int32_t* pool,
-                                    const InstDesc* insts, int count, int max_col, int max_n,
-                                    const double* A, double* LU, int32_t* status,
-                                    cudaStream_t stream);
+                                    const InstDesc* insts, const FlowBatch& b, const double* A,
+                                    double* LU, int32_t* status, cudaStream_t stream);
 bool complex_solve_in_smem(int max_n, const double* LU);
 cudaError_t launch_complex_solve(const PlanDesc* plans, const int32_t* pool, const InstDesc* insts,
-                                 int count, int max_n, const double* LU, double* X, double* W,
+                                 const FlowBatch& b, const double* LU, double* X, double* W,
                                  cudaStream_t stream);
 size_t complex_refactor_smem(int max_n);
 cudaError_t launch_grid_solve(const PlanDesc* plans, const int32_t* pool, const InstDesc* insts,
@@ -518,6 +518,14 @@ int nsg_topology_order_complex(int n, int nnz, const int* col_ptr, const int* ro
 
 void nsg_topology_free(nsg_topology* topo) { delete topo; }
 
+namespace {
+
+nsg::FlowBatch flow_batch(const nsg_batch& b) {
+    return {b.count, b.max_col, b.max_n, b.level_rows};
+}
+
+}  // namespace
+
 int nsg_batch_create(int count, nsg_topology* const* topos, nsg_batch** out) {
     return guarded("nsg_batch_create", [&]() -> int {
         if (!out || count <= 0 || !topos)
@@ -534,7 +542,7 @@ int nsg_batch_create(int count, nsg_topology* const* topos, nsg_batch** out) {
         b->a_off.assign(count + 1, 0);
         b->x_off.assign(count + 1, 0);
         b->lu_off.assign(count + 1, 0);
-        int64_t lrows = 0, urows = 0;
+        int64_t lrows = 0, urows = 0, levels = 0;
         for (int i = 0; i < count; ++i) {
             const nsg_topology* t = topos[i];
             if (!t) return fail(NSG_ERR_INVALID, "nsg_batch_create: null topology");
@@ -557,11 +565,13 @@ int nsg_batch_create(int count, nsg_topology* const* topos, nsg_batch** out) {
             insts[i].urows_off = urows;
             lrows += (p.lrow_ptr[p.n] + 3) & ~3;
             urows += (p.urow_ptr[p.n] + 3) & ~3;
+            levels += static_cast<int64_t>(p.fwd_lev_ptr.size()) - 1;
             b->a_off[i + 1] = b->a_off[i] + p.nnz_a;
             b->x_off[i + 1] = b->x_off[i] + p.n;
             // keep each instance's LU 32-byte aligned
             b->lu_off[i + 1] = b->lu_off[i] + ((p.nnz_lu + 3) & ~3);
         }
+        b->level_rows = static_cast<double>(b->x_off[count]) / std::max<double>(1, levels);
         // Largest instances first: the grid's tail is made of small ones.
         std::stable_sort(insts.begin(), insts.end(), [&](const nsg::InstDesc& x, const nsg::InstDesc& y) {
             return topos[x.index]->plan.updates > topos[y.index]->plan.updates;
@@ -605,8 +615,8 @@ int nsg_batch_refactor_complex(nsg_batch* b, const double* d_ax, double* d_lu, i
     if (smem > 200 * 1024)
         return fail(NSG_ERR_INVALID, "nsg_batch_refactor_complex: too many unknowns per instance "
                                      "for the shared-memory completion flags");
-    const cudaError_t e = nsg::launch_complex_refactor(b->d_plans, b->d_pool, b->d_insts, b->count,
-                                                       b->max_col, b->max_n, d_ax, d_lu, d_status,
+    const cudaError_t e = nsg::launch_complex_refactor(b->d_plans, b->d_pool, b->d_insts,
+                                                       flow_batch(*b), d_ax, d_lu, d_status,
                                                        static_cast<cudaStream_t>(stream));
     return e == cudaSuccess ? NSG_OK : cuda_fail("nsg_batch_refactor_complex", e);
 }
@@ -619,7 +629,7 @@ int nsg_batch_solve_complex(nsg_batch* b, const double* d_lu, double* d_x, void*
                        sizeof(double) * 2 * static_cast<size_t>(std::max<long long>(1, b->x_off[b->count])));
         if (e != cudaSuccess) return cuda_fail("nsg_batch_solve_complex: workspace", e);
     }
-    e = nsg::launch_complex_solve(b->d_plans, b->d_pool, b->d_insts, b->count, b->max_n, d_lu, d_x,
+    e = nsg::launch_complex_solve(b->d_plans, b->d_pool, b->d_insts, flow_batch(*b), d_lu, d_x,
                                   b->d_cwork, static_cast<cudaStream_t>(stream));
     return e == cudaSuccess ? NSG_OK : cuda_fail("nsg_batch_solve_complex", e);
 }
@@ -671,10 +681,10 @@ int nsg_batch_refactor(nsg_batch* b, const double* d_values, double diag_gmin,
         if (e == cudaSuccess) b->rows_valid = true;
         return e == cudaSuccess ? NSG_OK : cuda_fail("nsg_batch_refactor", e);
     }
-    cudaError_t e = nsg::launch_refactor(b->d_plans, b->d_pool, b->d_insts, b->count, d_values,
-                                         b->d_lu, diag_gmin, mode, 1e-3, d_status,
-                                         d_fail_step, b->max_col, b->max_n, b->allow_flow,
-                                         b->d_lrows, b->d_urows, static_cast<cudaStream_t>(stream));
+    cudaError_t e = nsg::launch_refactor(b->d_plans, b->d_pool, b->d_insts, flow_batch(*b),
+                                         d_values, b->d_lu, diag_gmin, mode, 1e-3, d_status,
+                                         d_fail_step, b->allow_flow, b->d_lrows, b->d_urows,
+                                         static_cast<cudaStream_t>(stream));
     if (e == cudaSuccess) b->rows_valid = b->allow_flow;
     return e == cudaSuccess ? NSG_OK : cuda_fail("nsg_batch_refactor", e);
 }
@@ -688,16 +698,16 @@ int nsg_batch_solve(nsg_batch* b, double* d_x, void* stream) {
                                                static_cast<cudaStream_t>(stream));
         return e == cudaSuccess ? NSG_OK : cuda_fail("nsg_batch_solve", e);
     }
-    cudaError_t e = nsg::launch_solve(b->d_plans, b->d_pool, b->d_insts, b->count, b->d_lu, d_x,
-                                      b->d_work, false, b->rows_valid ? b->d_lrows : nullptr,
-                                      b->d_urows, b->max_n, static_cast<cudaStream_t>(stream));
+    cudaError_t e = nsg::launch_solve(b->d_plans, b->d_pool, b->d_insts, flow_batch(*b), b->d_lu,
+                                      d_x, b->d_work, false, b->rows_valid ? b->d_lrows : nullptr,
+                                      b->d_urows, static_cast<cudaStream_t>(stream));
     return e == cudaSuccess ? NSG_OK : cuda_fail("nsg_batch_solve", e);
 }
 
 int nsg_batch_solve_transposed(nsg_batch* b, double* d_x, void* stream) {
     if (!b || !d_x) return fail(NSG_ERR_INVALID, "nsg_batch_solve_transposed: null argument");
-    cudaError_t e = nsg::launch_solve(b->d_plans, b->d_pool, b->d_insts, b->count, b->d_lu, d_x,
-                                      b->d_work, true, nullptr, nullptr, b->max_n,
+    cudaError_t e = nsg::launch_solve(b->d_plans, b->d_pool, b->d_insts, flow_batch(*b), b->d_lu,
+                                      d_x, b->d_work, true, nullptr, nullptr,
                                       static_cast<cudaStream_t>(stream));
     return e == cudaSuccess ? NSG_OK : cuda_fail("nsg_batch_solve_transposed", e);
 }

@@ -52,6 +52,7 @@ struct nsg_batch {
     bool rows_valid = false;    // the copies match d_lu (last refactor was dataflow)
     int max_col = 0;
     int max_n = 0;
+    double level_rows = 0.0;      // mean rows of a level of the triangular sweeps
     bool allow_flow = true;
     int schedule = 0;             // nsg_batch_set_schedule
     int grid_colbuf = 0;          // nsg_batch_set_grid_buffer (0: automatic)

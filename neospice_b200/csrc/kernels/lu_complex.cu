@@ -7,6 +7,7 @@
 // grouping (re = a*c - b*d, im = a*d + b*c, one rounding each), and every
 // entry receives its updates in ascending pivot order, so the factors and
 // solutions are bit-identical to the reference's under the same pivots.
+#include "flow_shape.cuh"
 #include "lu_cta.cuh"
 
 #include <cuda_runtime.h>
@@ -567,6 +568,7 @@ namespace {
 
 constexpr size_t kMaxCplxSmem = 200 * 1024;
 constexpr int kWideThreads = 512;
+constexpr int kRefactorNeed = 6, kSolveNeed = 4;  // flow_shape
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
@@ -582,61 +584,62 @@ cudaError_t launch_complex(Kernel kernel, int count, int threads, size_t smem, c
     return cudaGetLastError();
 }
 
-int cplx_sm_count() {
-    static const int sms = [] {
-        int dev = 0, n = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        return n > 0 ? n : 1;
-    }();
-    return sms;
+size_t complex_flow_bytes(int colbuf, int max_n, int warps) {
+    return sizeof(double2) * static_cast<size_t>(warps) * static_cast<size_t>(colbuf) +
+           sizeof(int32_t) * static_cast<size_t>(max_n);
+}
+size_t complex_sweep_bytes(int max_n) {
+    return (sizeof(double2) + sizeof(int32_t)) * static_cast<size_t>(max_n);
 }
 
 }  // namespace
 
-// One CTA of 16 warps per SM (128 registers a thread) for up to one instance
-// per SM, two (64 registers) for more.
 cudaError_t launch_complex_refactor(const PlanDesc* plans, const int32_t* pool,
-                                    const InstDesc* insts, int count, int max_col, int max_n,
-                                    const double* A, double* LU, int32_t* status,
-                                    cudaStream_t stream) {
-    const int colbuf = (max_col + 31) & ~31;
-    const size_t wide = sizeof(double2) * (kWideThreads / 32) * static_cast<size_t>(colbuf) +
-                        sizeof(int32_t) * static_cast<size_t>(max_n);
-    if (wide <= kMaxCplxSmem && aligned16(LU)) {
-        if (count <= cplx_sm_count())
-            return launch_complex(complex_flow_refactor_kernel<kWideThreads, 1>, count, kWideThreads,
-                                  wide, stream, plans, pool, insts, A, LU, status, colbuf);
-        return launch_complex(complex_flow_refactor_kernel<kWideThreads, 2>, count, kWideThreads,
-                              wide, stream, plans, pool, insts, A, LU, status, colbuf);
+                                    const InstDesc* insts, const FlowBatch& b, const double* A,
+                                    double* LU, int32_t* status, cudaStream_t stream) {
+    const int colbuf = (b.max_col + 31) & ~31;
+    if (complex_flow_bytes(colbuf, b.max_n, kWideThreads / 32) <= kMaxCplxSmem && aligned16(LU)) {
+        const FlowShape shape =
+            flow_shape(b, complex_flow_bytes(colbuf, b.max_n, kWideThreads / 64), kRefactorNeed);
+        const int threads = shape == kShapeMany ? kWideThreads / 2 : kWideThreads;
+        auto launch = [&](auto kernel) {
+            return launch_complex(kernel, b.count, threads,
+                                  complex_flow_bytes(colbuf, b.max_n, threads / 32), stream, plans,
+                                  pool, insts, A, LU, status, colbuf);
+        };
+        if (shape == kShapeAlone) return launch(complex_flow_refactor_kernel<kWideThreads, 1>);
+        if (shape == kShapePair) return launch(complex_flow_refactor_kernel<kWideThreads, 2>);
+        return launch(complex_flow_refactor_kernel<kWideThreads / 2, 4>);
     }
-    const size_t smem = complex_refactor_smem(max_n);
+    const size_t smem = complex_refactor_smem(b.max_n);
     if (smem > kUnaskedSmem) {
         const cudaError_t e = cudaFuncSetAttribute(
             complex_refactor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         if (e != cudaSuccess) return e;
     }
-    complex_refactor_kernel<<<count, kCplxThreads, smem, stream>>>(plans, pool, insts, A, LU,
-                                                                    status);
+    complex_refactor_kernel<<<b.count, kCplxThreads, smem, stream>>>(plans, pool, insts, A, LU,
+                                                                      status);
     return cudaGetLastError();
 }
 
 // Whether launch_complex_solve keeps the vector in shared memory (and needs no
 // workspace W).
 bool complex_solve_in_smem(int max_n, const double* LU) {
-    return (sizeof(double2) + sizeof(int32_t)) * static_cast<size_t>(max_n) <= kMaxCplxSmem &&
-           aligned16(LU);
+    return complex_sweep_bytes(max_n) <= kMaxCplxSmem && aligned16(LU);
 }
 
 cudaError_t launch_complex_solve(const PlanDesc* plans, const int32_t* pool, const InstDesc* insts,
-                                 int count, int max_n, const double* LU, double* X, double* W,
+                                 const FlowBatch& b, const double* LU, double* X, double* W,
                                  cudaStream_t stream) {
-    if (complex_solve_in_smem(max_n, LU)) {
-        const size_t smem = (sizeof(double2) + sizeof(int32_t)) * static_cast<size_t>(max_n);
-        return launch_complex(complex_flow_solve_kernel<kWideThreads, 2>, count, kWideThreads, smem,
+    if (complex_solve_in_smem(b.max_n, LU)) {
+        const size_t smem = complex_sweep_bytes(b.max_n);
+        if (flow_shape(b, smem, kSolveNeed) == kShapeMany)
+            return launch_complex(complex_flow_solve_kernel<kWideThreads / 2, 4>, b.count,
+                                  kWideThreads / 2, smem, stream, plans, pool, insts, LU, X);
+        return launch_complex(complex_flow_solve_kernel<kWideThreads, 2>, b.count, kWideThreads, smem,
                               stream, plans, pool, insts, LU, X);
     }
-    complex_solve_kernel<<<count, kCplxThreads, 0, stream>>>(plans, pool, insts, LU, X, W);
+    complex_solve_kernel<<<b.count, kCplxThreads, 0, stream>>>(plans, pool, insts, LU, X, W);
     return cudaGetLastError();
 }
 

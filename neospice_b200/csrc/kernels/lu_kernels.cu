@@ -13,6 +13,7 @@
 // at a time, with separately rounded multiply and subtract (__dmul_rn,
 // __dsub_rn: no FMA contraction).  Results are therefore bit-identical to the
 // reference under the same pivot sequence.
+#include "flow_shape.cuh"
 #include "lu_cta.cuh"
 
 #include <cuda_runtime.h>
@@ -211,25 +212,8 @@ solve_transposed_flow_kernel(const PlanDesc* __restrict__ plans, const int32_t* 
 
 namespace {
 
-// Launch shape of the dataflow kernels: one CTA of 16 warps with the SM's
-// registers to itself for up to one instance per SM, two such CTAs per SM for
-// up to twice that, else four CTAs of 8 warps, which keep as many warps busy
-// and twice the instances: with the run-wise refactor 592 refactors, solves and
-// transposed solves of 145 to 577 unknowns went from 778 us (two CTAs of 16
-// warps) to 670 us, one of 37 unknowns from 44.5 to 34.6 us.
-enum FlowShape { kShapeAlone, kShapePair, kShapeMany };
-
-FlowShape flow_shape(int count) {
-    static const int sms = [] {
-        int dev = 0, n = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        return n > 0 ? n : 1;
-    }();
-    return count <= sms ? kShapeAlone : count <= 2 * sms ? kShapePair : kShapeMany;
-}
-
 constexpr int kMaxFlowSmem = 200 * 1024;
+constexpr int kSolveNeed = 3;  // flow_shape
 
 template <class Kernel, class... Args>
 cudaError_t launch_flow(Kernel kernel, int count, int threads, size_t smem, cudaStream_t stream,
@@ -245,20 +229,23 @@ cudaError_t launch_flow(Kernel kernel, int count, int threads, size_t smem, cuda
 
 }  // namespace
 
-// max_col / max_n: largest LU column and order over the batch's plans.
 cudaError_t launch_refactor(const PlanDesc* plans, const int32_t* pool, const InstDesc* insts,
-                            int count, const double* A, double* LU, double diag_gmin,
+                            const FlowBatch& b, const double* A, double* LU, double diag_gmin,
                             int check_pivots, double rel_threshold, int32_t* status,
-                            int32_t* fail_step, int max_col, int max_n, bool allow_flow,
-                            double* lrows, double* urows, cudaStream_t stream) {
-    if (count <= 0) return cudaSuccess;
-    const int colbuf = (max_col + 31) & ~31;
-    if (allow_flow && flow_smem_bytes(colbuf, max_n) <= kMaxFlowSmem) {
-        const FlowShape shape = flow_shape(count);
+                            int32_t* fail_step, bool allow_flow, double* lrows, double* urows,
+                            cudaStream_t stream) {
+    if (b.count <= 0) return cudaSuccess;
+    const int colbuf = (b.max_col + 31) & ~31;
+    if (allow_flow && flow_smem_bytes(colbuf, b.max_n) <= kMaxFlowSmem) {
+        // three are enough where they hold the whole batch: 297 trees of 16,000
+        // unknowns 4.2 ms, on 16 warps 5.2; 592 trees 8.3 and 5.7
+        const int need = b.count <= 3 * flow_sm_count() ? 3 : 4;
+        const FlowShape shape =
+            flow_shape(b, flow_smem_bytes(colbuf, b.max_n, kFlowWarps / 2), need);
         const int threads = shape == kShapeMany ? kFlowThreads / 2 : kFlowThreads;
-        const size_t smem = flow_smem_bytes(colbuf, max_n, threads / 32);
+        const size_t smem = flow_smem_bytes(colbuf, b.max_n, threads / 32);
         auto launch = [&](auto kernel) {
-            return launch_flow(kernel, count, threads, smem, stream, plans, pool, insts, A, LU,
+            return launch_flow(kernel, b.count, threads, smem, stream, plans, pool, insts, A, LU,
                                diag_gmin, check_pivots, rel_threshold, status, fail_step, colbuf,
                                lrows, urows);
         };
@@ -266,26 +253,26 @@ cudaError_t launch_refactor(const PlanDesc* plans, const int32_t* pool, const In
         if (shape == kShapePair) return launch(refactor_flow_kernel<kFlowThreads, 2>);
         return launch(refactor_flow_kernel<kFlowThreads / 2, 4>);
     }
-    refactor_kernel<<<count, 256, 0, stream>>>(plans, pool, insts, A, LU, diag_gmin, check_pivots,
-                                               rel_threshold, status, fail_step);
+    refactor_kernel<<<b.count, 256, 0, stream>>>(plans, pool, insts, A, LU, diag_gmin,
+                                                 check_pivots, rel_threshold, status, fail_step);
     return cudaGetLastError();
 }
 
 cudaError_t launch_solve(const PlanDesc* plans, const int32_t* pool, const InstDesc* insts,
-                         int count, const double* LU, double* X, double* W, bool transposed,
-                         const double* lrows, const double* urows, int max_n,
+                         const FlowBatch& b, const double* LU, double* X, double* W,
+                         bool transposed, const double* lrows, const double* urows,
                          cudaStream_t stream) {
-    if (count <= 0) return cudaSuccess;
-    const size_t smem = flow_solve_smem_bytes(max_n);
+    if (b.count <= 0) return cudaSuccess;
+    const size_t smem = flow_solve_smem_bytes(b.max_n);
     if ((transposed || lrows) && smem <= kMaxFlowSmem) {
-        const FlowShape shape = flow_shape(count);
+        const FlowShape shape = flow_shape(b, smem, kSolveNeed);
         const int threads = shape == kShapeMany ? kFlowThreads / 2 : kFlowThreads;
         auto forward = [&](auto kernel) {
-            return launch_flow(kernel, count, threads, smem, stream, plans, pool, insts, LU, lrows,
+            return launch_flow(kernel, b.count, threads, smem, stream, plans, pool, insts, LU, lrows,
                                urows, X);
         };
         auto back = [&](auto kernel) {
-            return launch_flow(kernel, count, threads, smem, stream, plans, pool, insts, LU, X);
+            return launch_flow(kernel, b.count, threads, smem, stream, plans, pool, insts, LU, X);
         };
         if (shape == kShapeMany)
             return transposed ? back(solve_transposed_flow_kernel<kFlowThreads / 2, 4>)
@@ -294,9 +281,9 @@ cudaError_t launch_solve(const PlanDesc* plans, const int32_t* pool, const InstD
                           : forward(solve_flow_kernel<kFlowThreads, 2>);
     }
     if (transposed)
-        solve_transposed_kernel<<<count, 256, 0, stream>>>(plans, pool, insts, LU, X, W);
+        solve_transposed_kernel<<<b.count, 256, 0, stream>>>(plans, pool, insts, LU, X, W);
     else
-        solve_kernel<<<count, 256, 0, stream>>>(plans, pool, insts, LU, X, W);
+        solve_kernel<<<b.count, 256, 0, stream>>>(plans, pool, insts, LU, X, W);
     return cudaGetLastError();
 }
 

@@ -1,0 +1,92 @@
+// Launch shapes of a batch's dataflow kernels without a GPU: the library's own
+// launch functions run against stand-ins for the runtime calls they make.
+// Prints "0 failure(s)" on success.
+#include "kernels/flow_shape.cuh"
+#include "kernels/lu_device.cuh"
+
+#include <cuda_runtime.h>
+
+#include <cstdint>
+#include <cstdio>
+
+namespace {
+int threads = 0, failures = 0;
+
+void expect(const char* what, int n, int count, int want) {
+    if (threads != want && ++failures < 20)
+        std::printf("failed: %s of %d, %d instances: %d threads\n", what, n, count, threads);
+}
+}  // namespace
+
+extern "C" {
+cudaError_t cudaGetDevice(int* d) { return *d = 0, cudaSuccess; }
+cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int) { return *v = 148, cudaSuccess; }
+cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaFuncSetAttribute(const void*, cudaFuncAttribute, int) { return cudaSuccess; }
+cudaError_t cudaLaunchKernel(const void*, dim3, dim3 block, void**, size_t, cudaStream_t) {
+    threads = static_cast<int>(block.x);
+    return cudaSuccess;
+}
+}
+
+namespace nsg {
+bool register_wait_limit_setter(cudaError_t (*)(int)) { return true; }
+cudaError_t launch_refactor(const PlanDesc*, const int32_t*, const InstDesc*, const FlowBatch&,
+                            const double*, double*, double, int, double, int32_t*, int32_t*, bool,
+                            double*, double*, cudaStream_t);
+cudaError_t launch_solve(const PlanDesc*, const int32_t*, const InstDesc*, const FlowBatch&,
+                         const double*, double*, double*, bool, const double*, const double*,
+                         cudaStream_t);
+cudaError_t launch_complex_refactor(const PlanDesc*, const int32_t*, const InstDesc*,
+                                    const FlowBatch&, const double*, double*, int32_t*,
+                                    cudaStream_t);
+cudaError_t launch_complex_solve(const PlanDesc*, const int32_t*, const InstDesc*,
+                                 const FlowBatch&, const double*, double*, double*, cudaStream_t);
+}  // namespace nsg
+
+namespace {
+
+const double* const kRows = reinterpret_cast<const double*>(64);
+double* const kLu = reinterpret_cast<double*>(64);
+
+void check(int n, int col, double level_rows, int refactor, int solve, int complex_refactor,
+           int complex_solve) {
+    for (int count : {1, 148, 149, 296, 297, 444, 445, 592, 1500}) {
+        const nsg::FlowBatch b{count, col, n, level_rows};
+        auto want = [&](int many) { return count <= 296 ? 512 : many; };
+        nsg::launch_refactor(nullptr, nullptr, nullptr, b, nullptr, kLu, 0.0, 0, 0.0, nullptr,
+                             nullptr, true, nullptr, nullptr, nullptr);
+        // three CTAs do where they hold the whole batch
+        const bool three = nsg::ctas_per_sm(8 * 8 * ((col + 31) / 32 * 32) + 4 * n) == 3;
+        expect("refactor", n, count, three && count <= 444 ? want(256) : want(refactor));
+        for (bool transposed : {false, true}) {
+            nsg::launch_solve(nullptr, nullptr, nullptr, b, kLu, nullptr, nullptr, transposed,
+                              transposed ? nullptr : kRows, kRows, nullptr);
+            expect(transposed ? "transposed solve" : "solve", n, count, want(solve));
+        }
+        nsg::launch_complex_refactor(nullptr, nullptr, nullptr, b, nullptr, kLu, nullptr, nullptr);
+        expect("complex refactor", n, count, want(complex_refactor));
+        nsg::launch_complex_solve(nullptr, nullptr, nullptr, b, kLu, nullptr, nullptr, nullptr);
+        expect("complex solve", n, count, want(complex_solve));
+    }
+}
+
+}  // namespace
+
+int main() {
+    // meshes (rows of a level from 2.5 to 20), at the sizes where fewer CTAs fit
+    check(37, 12, 2.5, 256, 256, 256, 256);
+    check(1601, 96, 10.0, 256, 256, 256, 256);
+    check(2816, 352, 15.0, 256, 256, 512, 256);  // complex vector: four CTAs up to 2816
+    check(2817, 192, 15.0, 256, 256, 256, 512);
+    check(6314, 224, 15.0, 256, 256, 512, 512);  // vector and flags: three CTAs up to 6314
+    check(6315, 224, 15.0, 256, 512, 512, 512);
+    check(8101, 448, 18.0, 512, 512, 512, 512);    // three refactors
+    check(10000, 600, 20.0, 512, 512, 512, 512);   // two
+    // chains
+    check(300, 2, 1.0, 256, 256, 256, 256);
+    check(9000, 13, 1.0, 256, 256, 256, 256);
+    check(10000, 2, 1.0, 256, 256, 256, 256);
+    std::printf("%d failure(s)\n", failures);
+    return failures == 0 ? 0 : 1;
+}
