@@ -479,8 +479,8 @@ complex_refactor_kernel(const PlanDesc* __restrict__ plans, const int32_t* __res
 // each accumulating its updates in the reference's order (forward: columns
 // ascending, skipping zero x_c; backward: row dot in ascending column order).
 // w: 2n doubles of scratch.
-__device__ __noinline__ void c_solve_levels(const PlanDesc& pd, const int32_t* pool,
-                                            const double* lu, double* x, double* w) {
+__device__ __forceinline__ void c_solve_rows(const PlanDesc& pd, const int32_t* pool,
+                                             const double* lu, double* x, double* w) {
     const int32_t n = pd.n;
     const int32_t* perm_row = pool + pd.off[PA_perm_row];
     const int32_t* perm_col = pool + pd.off[PA_perm_col];
@@ -550,13 +550,20 @@ __device__ __noinline__ void c_solve_levels(const PlanDesc& pd, const int32_t* p
     }
 }
 
+// The same out of line, for the kernel that reaches it only where a bounded wait
+// gave up.
+__device__ __noinline__ void c_solve_levels(const PlanDesc& pd, const int32_t* pool,
+                                            const double* lu, double* x, double* w) {
+    c_solve_rows(pd, pool, lu, x, w);
+}
+
 // The general solve (as the general refactor), one instance per CTA.
 __global__ void __launch_bounds__(kCplxThreads)
 complex_solve_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restrict__ pool,
                      const InstDesc* __restrict__ insts, const double* __restrict__ LU,
                      double* X, double* W) {
     const InstDesc id = insts[blockIdx.x];
-    c_solve_levels(plans[id.plan], pool, LU + 2 * id.lu_off, X + 2 * id.x_off, W + 2 * id.w_off);
+    c_solve_rows(plans[id.plan], pool, LU + 2 * id.lu_off, X + 2 * id.x_off, W + 2 * id.w_off);
 }
 
 }  // namespace
