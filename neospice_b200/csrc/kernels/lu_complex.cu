@@ -342,6 +342,10 @@ complex_flow_solve_kernel(const PlanDesc* __restrict__ plans, const int32_t* __r
     const int32_t* diag_pos = pool + pd.off[PA_diag_pos];
     const double2* lu = reinterpret_cast<const double2*>(LU) + id.lu_off;
     double* x = X + 2 * id.x_off;
+    if (wide_levels(pd)) {
+        c_solve_levels(pd, pool, LU + 2 * id.lu_off, x, reinterpret_cast<double*>(cols));
+        return;
+    }
     volatile int32_t* done = reinterpret_cast<volatile int32_t*>(cols + n);
     __shared__ int32_t s_ok;
     if (threadIdx.x == 0) s_ok = 1;
@@ -550,8 +554,8 @@ __device__ __forceinline__ void c_solve_rows(const PlanDesc& pd, const int32_t* 
     }
 }
 
-// The same out of line, for the kernel that reaches it only where a bounded wait
-// gave up.
+// The same out of line, for the kernel that reaches it only for wide levels or
+// where a bounded wait gave up.
 __device__ __noinline__ void c_solve_levels(const PlanDesc& pd, const int32_t* pool,
                                             const double* lu, double* x, double* w) {
     c_solve_rows(pd, pool, lu, x, w);

@@ -639,8 +639,8 @@ __device__ inline void cta_solve(const PlanDesc& pd, const int32_t* __restrict__
     __syncthreads();
 }
 
-// cta_solve out of line, for kernels that reach it only where a bounded wait of
-// their dataflow sweeps gave up.
+// cta_solve out of line, for kernels that reach it only for wide levels or where a
+// bounded wait of their dataflow sweeps gave up.
 static __device__ __noinline__ void cta_solve_levels(const PlanDesc& pd,
                                                      const int32_t* __restrict__ pool,
                                                      const double* __restrict__ lu,
@@ -1271,6 +1271,10 @@ static __device__ __noinline__ bool cta_solve_flow(const PlanDesc& pd, const int
                                       const double* __restrict__ lrows,
                                       const double* __restrict__ urows, double* __restrict__ x,
                                       double* smem) {
+    if (wide_levels(pd)) {
+        cta_solve_levels(pd, pool, lu, x, smem);
+        return true;
+    }
     const int32_t n = pd.n;
     const bool amd = pd.kind == kPlanAmdLu;
     const int32_t* lp = pool + pd.off[PA_lrow_ptr];
@@ -1310,6 +1314,10 @@ static __device__ __noinline__ void cta_solve_transposed_flow(const PlanDesc& pd
                                                               const double* __restrict__ lu,
                                                               double* __restrict__ x,
                                                               double* smem) {
+    if (wide_levels(pd)) {
+        cta_solve_transposed_levels(pd, pool, lu, x, smem);
+        return;
+    }
     const int32_t n = pd.n;
     const bool amd = pd.kind == kPlanAmdLu;
     const int32_t* cp = pool + pd.off[PA_col_ptr];

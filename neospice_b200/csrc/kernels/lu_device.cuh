@@ -32,6 +32,22 @@ struct PlanDesc {
     const int32_t* lp_at;
 };
 
+// Whether a plan's levels hold so many rows for the entries of each that a thread
+// per row and a barrier per level solve it faster than a warp per row: 16 times
+// as many rows in a level as entries in a row (an interconnect tree of random
+// branches: one entry, 10 rows a level at 100 unknowns, 500 at 10,000; meshes,
+// bands and chains at most 2 rows per entry).  A warp has one lane at work in a row
+// of one entry: 592 solves of 1502-unknown trees took 0.27 ms, 0.07 here, of
+// 10,002 5.2 and 0.58 ms, one transient of 3000 nodes 100 and 80 ms; 592 of 102
+// unknowns (10 rows a level, a warp per row) 0.04 ms either way.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline bool wide_levels(const PlanDesc& pd) {
+    const long long n = pd.n;
+    return 8LL * (pd.nnz_lu - pd.n) * pd.n_fwd_lev <= n * n;
+}
+
 #ifdef __CUDACC__
 // Entry k of a plan's update map: the position in column j that update k
 // of U(r, j) writes.  Packed plans (map16) hold it in 16 bits, halving the

@@ -1,6 +1,6 @@
 // Launch shapes of a batch's dataflow kernels without a GPU: the library's own
 // launch functions run against stand-ins for the runtime calls they make.
-// Prints "0 failure(s)" on success.
+// And which plans are solved with a thread per row.  Prints "0 failure(s)" on success.
 #include "kernels/flow_shape.cuh"
 #include "kernels/lu_device.cuh"
 
@@ -71,6 +71,18 @@ void check(int n, int col, double level_rows, int refactor, int solve, int compl
     }
 }
 
+// n unknowns, off-diagonal entries a row of a sweep, rows a level
+void wide(int n, double entries, double level_rows, bool want) {
+    nsg::PlanDesc pd{};
+    pd.n = n;
+    pd.nnz_lu = n + static_cast<int>(2 * entries * n);
+    pd.n_fwd_lev = static_cast<int>(n / level_rows);
+    if (nsg::wide_levels(pd) != want) {
+        std::printf("failed: %d unknowns, %g entries, %g rows\n", n, entries, level_rows);
+        ++failures;
+    }
+}
+
 }  // namespace
 
 int main() {
@@ -87,6 +99,16 @@ int main() {
     check(300, 2, 1.0, 256, 256, 256, 256);
     check(9000, 13, 1.0, 256, 256, 256, 256);
     check(10000, 2, 1.0, 256, 256, 256, 256);
+    wide(10002, 1.0, 500.0, true);  // trees of random branches
+    wide(502, 1.0, 36.0, true);
+    wide(202, 1.0, 16.8, true);
+    wide(202, 1.0, 15.0, false);
+    wide(1, 0.0, 1.0, true);        // no entries at all
+    wide(3000, 1.0, 10.0, false);   // a tree of short branches
+    wide(10000, 1.0, 1.0, false);   // a chain
+    wide(16385, 24.0, 21.0, false); // meshes
+    wide(37, 3.4, 2.5, false);
+    wide(20000000, 25.0, 20.0, false);
     std::printf("%d failure(s)\n", failures);
     return failures == 0 ? 0 : 1;
 }

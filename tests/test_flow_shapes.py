@@ -1,6 +1,7 @@
 """The launch functions of a batch's refactors and solves against stand-ins for the
 CUDA runtime (tests/cpp/flow_shape_check.cpp, linked here with the library's
-own objects): the shape follows what fits an SM, not the instance count alone."""
+own objects): the shape follows what fits an SM, not the instance count alone.  And
+which plans are solved with a thread per row."""
 import pathlib
 import subprocess
 
