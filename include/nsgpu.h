@@ -246,7 +246,9 @@ int nsg_batch_refactor_complex(nsg_batch* batch, const double* d_ax, double* d_l
                                void* stream);
 /* SparseMatrix::solve_complex (src/solver/solve.cpp:49-100) on d_lu: d_x
  * holds b on entry and x on return, interleaved, 2*vector_offsets per
- * instance.  The first call allocates the batch's complex sweep workspace. */
+ * instance.  The vectors are kept in shared memory up to 10,240 unknowns and for
+ * a d_lu that is 16-byte aligned; else the first call allocates the batch's
+ * complex sweep workspace. */
 int nsg_batch_solve_complex(nsg_batch* batch, const double* d_lu, double* d_x, void* stream);
 
 /* Device pointer to the factored LU values (layout per nsg_batch_layout and
@@ -546,10 +548,13 @@ int nsg_tran_batch_create(int count, nsg_circuit* const* circuits, double tstep,
 void nsg_tran_batch_free(nsg_tran_batch* b);
 /* Launch shape of the transient kernel: threads per CTA (128, 256 or 512)
  * and CTAs per SM (128: 8; 256: 4; 512: 2; 0 = that default), or 0, 0 for
- * the automatic choice (512 for any instance above 128 unknowns; else 128
- * or 256, enough for one pass of the device loads, four or two CTAs per
- * SM, one for up to one instance per SM).  Tuning only: the shapes give the same results.  No counterpart
- * in the reference. */
+ * the automatic choice, which has shapes of its own: 512 threads, one or two
+ * CTAs per SM, where an instance has more than 128 unknowns, more than 256
+ * devices of a family or a factor for the dataflow kernels; else 256 threads,
+ * one CTA per SM, for up to one instance per SM, and for more 128 threads, four
+ * CTAs, or 256, two (more than 128 devices of a family, or level programs that
+ * four CTAs have no room for).  Tuning only: the shapes give the same results.
+ * No counterpart in the reference. */
 int nsg_tran_batch_set_shape(nsg_tran_batch* b, int threads, int blocks_per_sm);
 /* Run the whole batch on a stream.  Instances stop for the host when a
  * solver needs ordering -- the transient solver on the first transient

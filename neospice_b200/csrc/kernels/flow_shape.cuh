@@ -15,7 +15,8 @@ struct FlowBatch {
 };
 
 // One CTA of 16 warps with the SM's registers to itself, two such CTAs, or four
-// of 8 warps.
+// of 8 warps.  (The sweeps need no more than 64 registers a thread: one
+// kernel serves the first two.)
 enum FlowShape { kShapeAlone, kShapePair, kShapeMany };
 
 inline int flow_sm_count() {

@@ -682,9 +682,9 @@ inline size_t stage_bytes_for(size_t scratch_bytes, const int64_t* lens, int cou
 // steps (a right-hand side is one more column).
 // Measured on a B200 at 1965 MHz: refactor and solve of the 32-stage inverter
 // chain 77,000 -> 17,800 cycles a Newton iteration (the steps 12,500 of them);
-// one transient of it (0.3 ns) 50.3 -> 25.0 ms, 300 BSIM4v7 ring + NAND
-// instances (0.06 ns) 224 -> 103 ms, transient and adjoint of 64 500-node
-// trees (0.1 ns) 119 -> 34.5 ms.
+// a pass of one transient of it (0.3 ns) 50.3 -> 25.0 ms, of 300 BSIM4v7 ring +
+// NAND instances (0.06 ns) 224 -> 103 ms, of transient and adjoint of 64
+// 500-node trees (0.1 ns) 119 -> 34.5 ms, all in CTAs of 512 threads.
 // Every entry applies its updates in the order of the column-wise refactor,
 // with the same rounded operations, so all values are bit-identical.
 // The space: pd.nnz_lu LU values, the vector (pd.n), the unscaled pivots (pd.n),

@@ -371,8 +371,9 @@ __device__ __forceinline__ double sum_terms_warp(const int32_t* terms, int32_t b
 // per matrix slot or rhs row, the rows beside the slots.  Lists longer than
 // kAsmLong (a supply node's, with terms of every device on it) are summed by
 // the whole warp, one after another.  One load after another, a thread took
-// two memory round trips a term: 400 inverter chains 55.0 -> 51.5 ms, 300
-// BSIM4v7 ring + NAND instances 108 -> 99 ms.
+// two memory round trips a term: a pass of 400 inverter chains (0.2 ns) 55.0 ->
+// 51.5 ms, of 300 BSIM4v7 ring + NAND instances (0.06 ns) 108 -> 99 ms, both
+// with two CTAs of 512 threads per SM.
 constexpr int32_t kAsmLong = 24;
 static __device__ __noinline__ void assemble(const Inst& v) {
     const int lane = threadIdx.x & 31;

@@ -583,11 +583,12 @@ size_t tran_smem_bytes(int max_col, int max_n) {
 //                               have no room for the level programs
 // else CTAs of 512 threads, one per SM (128 registers) or two (64): a factor on
 // the dataflow kernels keeps their 16 warps busy.
-// Passes measured on a B200, two CTAs of 512 threads per SM (small batches) or
-// 1024 threads per SM (large ones) -> these: one inverter chain 25.8 -> 20.4
-// ms, 400 chains 37.3 -> 35.4, 1184 chains 94.7 -> 94.3; BSIM4v7 ring + NAND,
-// 300 instances 79.3 -> 69.2, 1184 instances 224 -> 197 ms; transient and
-// adjoint of 64 500-node trees 32.9 -> 27.9 ms.
+// Whole passes (nsg_tran_batch_run again on the same batch, host rounds included)
+// on a B200 at 1965 MHz, against the shapes that can be asked for: 32-stage
+// inverter chains, 0.3 ns: one 20.2 ms (512 threads, two per SM: 24.6), 400
+// 55.6 (75.4; 128 threads, eight: 60.2), 1184 140 (137; 256 threads, four: 152);
+// BSIM4v7 ring + NAND, 0.06 ns: 300 instances 74.9 (82.8; 87.5), 1184 226 (256
+// threads, four: 261).
 // sh.force_threads / force_blocks (0: automatic) override the choice.
 cudaError_t launch_transient(const PlanDesc* plans, const int32_t* lu_pool, const DcDesc* descs,
                              const TranDesc* tdescs, const int32_t* subset, int count,
