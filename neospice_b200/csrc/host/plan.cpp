@@ -361,10 +361,10 @@ void finish(TopologyPlan& p) {
 }  // namespace
 
 // The level program of a Markowitz plan (see TopologyPlan::lp), for factors
-// within the bounds above that have an update map.  An entry of the factor receives its updates in
-// ascending pivot order, a row of a sweep its columns in the order of the
-// row-wise sweeps, so every value is the one the column-wise refactor and the
-// sweeps compute.
+// within the bounds above that have an update map.  An entry of the factor
+// receives its updates in ascending pivot order, a row of a sweep its columns in
+// the order of the row-wise sweeps, so every value is the one the column-wise
+// refactor and the sweeps compute.
 void build_level_program(TopologyPlan& p) {
     p.lp.clear();
     p.lp_core = 0;

@@ -214,8 +214,8 @@ TopologyPlan build_plan(const MarkowitzOrder& mo, const std::vector<int32_t>& sl
 TopologyPlan build_plan_amd(const AmdLuFactor& f);
 
 // Give a plan its level program (TopologyPlan::lp) if it is a small sparse
-// Markowitz plan with an update map; clears it otherwise.  The batches of circuits call it for
-// each distinct plan they keep.
+// Markowitz plan with an update map; clears it otherwise.  The batches of
+// circuits call it for each distinct plan they keep.
 void build_level_program(TopologyPlan& p);
 
 // Build from an exported structure (the reference's own NeoSolver state):
