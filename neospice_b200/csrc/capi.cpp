@@ -521,7 +521,7 @@ void nsg_topology_free(nsg_topology* topo) { delete topo; }
 namespace {
 
 nsg::FlowBatch flow_batch(const nsg_batch& b) {
-    return {b.count, b.max_col, b.max_n, b.level_rows};
+    return {b.count, b.max_col, b.max_n, b.level_rows, b.wide};
 }
 
 }  // namespace
@@ -550,6 +550,7 @@ int nsg_batch_create(int count, nsg_topology* const* topos, nsg_batch** out) {
             if (it == plan_of.end()) {
                 it = plan_of.emplace(t, static_cast<int32_t>(plans.size())).first;
                 plans.push_back(make_plan_desc(t->plan, pool));
+                b->wide = b->wide || nsg::wide_levels(plans.back());
             }
             const auto& p = t->plan;
             if (!p.has_update_map) b->unmapped = true;

@@ -53,6 +53,7 @@ struct nsg_batch {
     int max_col = 0;
     int max_n = 0;
     double level_rows = 0.0;      // mean rows of a level of the triangular sweeps
+    bool wide = false;            // a plan has wide levels (nsg::wide_levels)
     bool allow_flow = true;
     int schedule = 0;             // nsg_batch_set_schedule
     int grid_colbuf = 0;          // nsg_batch_set_grid_buffer (0: automatic)

@@ -7,11 +7,13 @@
 
 namespace nsg {
 
-// What the shapes depend on: instances, the batch's largest LU column and
-// order, and the mean number of rows in a level of its triangular sweeps.
+// What the launches depend on: instances, the batch's largest LU column and
+// order, the mean number of rows in a level of its triangular sweeps, and whether
+// any plan has wide levels (wide_levels).
 struct FlowBatch {
     int count = 0, max_col = 0, max_n = 0;
     double level_rows = 0.0;
+    bool wide = false;
 };
 
 // One CTA of 16 warps with the SM's registers to itself, two such CTAs, or four

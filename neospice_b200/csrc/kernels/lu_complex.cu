@@ -332,7 +332,7 @@ template <int kThreads, int kBlocks>
 __global__ void __launch_bounds__(kThreads, kBlocks)
 complex_flow_solve_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restrict__ pool,
                           const InstDesc* __restrict__ insts, const double* __restrict__ LU,
-                          double* X) {
+                          double* X, bool any_wide) {
     extern __shared__ __align__(16) double2 cols[];
     const InstDesc id = insts[blockIdx.x];
     const PlanDesc& pd = plans[id.plan];
@@ -342,7 +342,7 @@ complex_flow_solve_kernel(const PlanDesc* __restrict__ plans, const int32_t* __r
     const int32_t* diag_pos = pool + pd.off[PA_diag_pos];
     const double2* lu = reinterpret_cast<const double2*>(LU) + id.lu_off;
     double* x = X + 2 * id.x_off;
-    if (wide_levels(pd)) {
+    if (any_wide && wide_levels(pd)) {
         c_solve_levels(pd, pool, LU + 2 * id.lu_off, x, reinterpret_cast<double*>(cols));
         return;
     }
@@ -646,9 +646,9 @@ cudaError_t launch_complex_solve(const PlanDesc* plans, const int32_t* pool, con
         const size_t smem = complex_sweep_bytes(b.max_n);
         if (flow_shape(b, smem, kSolveNeed) == kShapeMany)
             return launch_complex(complex_flow_solve_kernel<kWideThreads / 2, 4>, b.count,
-                                  kWideThreads / 2, smem, stream, plans, pool, insts, LU, X);
+                                  kWideThreads / 2, smem, stream, plans, pool, insts, LU, X, b.wide);
         return launch_complex(complex_flow_solve_kernel<kWideThreads, 2>, b.count, kWideThreads, smem,
-                              stream, plans, pool, insts, LU, X);
+                              stream, plans, pool, insts, LU, X, b.wide);
     }
     complex_solve_kernel<<<b.count, kCplxThreads, 0, stream>>>(plans, pool, insts, LU, X, W);
     return cudaGetLastError();

@@ -1265,13 +1265,15 @@ __device__ __forceinline__ bool sweep_pair(int32_t n, const int32_t* perm_in,
 // x <- A^{-1} x (SparseMatrix::solve) by the whole CTA: L forward with the
 // reciprocal pivot, U backward (AMD-LU: unit L, then U columns descending and
 // the pivot division), on the row-major copies the refactor wrote.  Same
-// arithmetic, in the same order per row, as cta_solve.
+// arithmetic, in the same order per row, as cta_solve.  any_wide: false where no
+// plan of the launch has wide levels, which saves the look at the plan (0.2 of a
+// 37-unknown refactor and solve's 34.7 us).
 static __device__ __noinline__ bool cta_solve_flow(const PlanDesc& pd, const int32_t* __restrict__ pool,
                                       const double* __restrict__ lu,
                                       const double* __restrict__ lrows,
                                       const double* __restrict__ urows, double* __restrict__ x,
-                                      double* smem) {
-    if (wide_levels(pd)) {
+                                      double* smem, bool any_wide = true) {
+    if (any_wide && wide_levels(pd)) {
         cta_solve_levels(pd, pool, lu, x, smem);
         return true;
     }
@@ -1313,8 +1315,9 @@ static __device__ __noinline__ void cta_solve_transposed_flow(const PlanDesc& pd
                                                               const int32_t* __restrict__ pool,
                                                               const double* __restrict__ lu,
                                                               double* __restrict__ x,
-                                                              double* smem) {
-    if (wide_levels(pd)) {
+                                                              double* smem,
+                                                              bool any_wide = true) {
+    if (any_wide && wide_levels(pd)) {
         cta_solve_transposed_levels(pd, pool, lu, x, smem);
         return;
     }

@@ -182,11 +182,11 @@ __global__ void __launch_bounds__(kThreads, kBlocks)
 solve_flow_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restrict__ pool,
                   const InstDesc* __restrict__ insts, const double* __restrict__ LU,
                   const double* __restrict__ lrows, const double* __restrict__ urows,
-                  double* __restrict__ X) {
+                  double* __restrict__ X, bool any_wide) {
     extern __shared__ double smem[];
     const InstDesc inst = insts[blockIdx.x];
     if (!cta_solve_flow(plans[inst.plan], pool, LU + inst.lu_off, lrows + inst.lrows_off,
-                        urows + inst.urows_off, X + inst.x_off, smem))
+                        urows + inst.urows_off, X + inst.x_off, smem, any_wide))
         cta_solve_levels(plans[inst.plan], pool, LU + inst.lu_off, X + inst.x_off, smem);
 }
 
@@ -204,10 +204,11 @@ template <int kThreads, int kBlocks>
 __global__ void __launch_bounds__(kThreads, kBlocks)
 solve_transposed_flow_kernel(const PlanDesc* __restrict__ plans, const int32_t* __restrict__ pool,
                              const InstDesc* __restrict__ insts, const double* __restrict__ LU,
-                             double* __restrict__ X) {
+                             double* __restrict__ X, bool any_wide) {
     extern __shared__ double smem[];
     const InstDesc inst = insts[blockIdx.x];
-    cta_solve_transposed_flow(plans[inst.plan], pool, LU + inst.lu_off, X + inst.x_off, smem);
+    cta_solve_transposed_flow(plans[inst.plan], pool, LU + inst.lu_off, X + inst.x_off, smem,
+                              any_wide);
 }
 
 namespace {
@@ -269,10 +270,11 @@ cudaError_t launch_solve(const PlanDesc* plans, const int32_t* pool, const InstD
         const int threads = shape == kShapeMany ? kFlowThreads / 2 : kFlowThreads;
         auto forward = [&](auto kernel) {
             return launch_flow(kernel, b.count, threads, smem, stream, plans, pool, insts, LU, lrows,
-                               urows, X);
+                               urows, X, b.wide);
         };
         auto back = [&](auto kernel) {
-            return launch_flow(kernel, b.count, threads, smem, stream, plans, pool, insts, LU, X);
+            return launch_flow(kernel, b.count, threads, smem, stream, plans, pool, insts, LU, X,
+                               b.wide);
         };
         if (shape == kShapeMany)
             return transposed ? back(solve_transposed_flow_kernel<kFlowThreads / 2, 4>)
