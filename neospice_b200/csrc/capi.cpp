@@ -24,6 +24,7 @@ cudaError_t launch_refactor(const PlanDesc* plans, const int32_t* pool, const In
                             int check_pivots, double rel_threshold, int32_t* status,
                             int32_t* fail_step, bool allow_flow, double* lrows, double* urows,
                             cudaStream_t stream);
+bool transposed_levels_pay(const FlowBatch& b);
 cudaError_t launch_solve(const PlanDesc* plans, const int32_t* pool, const InstDesc* insts,
                          const FlowBatch& b, const double* LU, double* X, double* W,
                          bool transposed, const double* lrows, const double* urows,
@@ -41,6 +42,7 @@ cudaError_t launch_complex_refactor(const PlanDesc* plans, const int32_t* pool,
                                     const InstDesc* insts, const FlowBatch& b, const double* A,
                                     double* LU, int32_t* status, cudaStream_t stream);
 bool complex_solve_in_smem(int max_n, const double* LU);
+bool complex_levels_pay(const FlowBatch& b, const double* LU);
 cudaError_t launch_complex_solve(const PlanDesc* plans, const int32_t* pool, const InstDesc* insts,
                                  const FlowBatch& b, const double* LU, double* X, double* W,
                                  cudaStream_t stream);
@@ -521,8 +523,51 @@ void nsg_topology_free(nsg_topology* topo) { delete topo; }
 namespace {
 
 nsg::FlowBatch flow_batch(const nsg_batch& b) {
-    return {b.count, b.max_col, b.max_n, b.level_rows, b.wide};
+    return {b.count, b.max_col, b.max_n, b.level_rows, b.row_entries, b.wide};
 }
+
+// The batch's pool, if a call may want a workspace of its own: memory once taken
+// stays with it.  Without one (an error is not passed on) no call does.
+void create_pool(nsg_batch& b) {
+    const nsg::FlowBatch fb = flow_batch(b);
+    if (!nsg::transposed_levels_pay(fb) && !nsg::complex_levels_pay(fb, nullptr)) return;
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location = {cudaMemLocationTypeDevice, b.device};
+    uint64_t keep = ~uint64_t{0};
+    if (cudaMemPoolCreate(&b.pool, &props) == cudaSuccess &&
+        cudaMemPoolSetAttribute(b.pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess)
+        return;
+    if (b.pool) cudaMemPoolDestroy(b.pool);
+    b.pool = nullptr;
+    cudaGetLastError();
+}
+
+// Device memory for one call on a stream, from the batch's pool and given back in
+// the stream's order, so calls on several streams or threads each have their
+// own.  None (null) where there is no memory, and while the stream is captured:
+// a graph with memory nodes could not be a child of another.
+class StreamScratch {
+public:
+    StreamScratch(const nsg_batch& b, size_t bytes, cudaStream_t st) : st_(st) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
+        if (!b.pool || cudaStreamIsCapturing(st, &cap) != cudaSuccess ||
+            (cap == cudaStreamCaptureStatusNone &&
+             cudaMallocFromPoolAsync(&p_, bytes, b.pool, st) != cudaSuccess)) {
+            p_ = nullptr;
+            cudaGetLastError();
+        }
+    }
+    StreamScratch(const StreamScratch&) = delete;
+    ~StreamScratch() {
+        if (p_) cudaFreeAsync(p_, st_);
+    }
+    double* data() const { return static_cast<double*>(p_); }
+
+private:
+    cudaStream_t st_;
+    void* p_ = nullptr;
+};
 
 }  // namespace
 
@@ -542,7 +587,7 @@ int nsg_batch_create(int count, nsg_topology* const* topos, nsg_batch** out) {
         b->a_off.assign(count + 1, 0);
         b->x_off.assign(count + 1, 0);
         b->lu_off.assign(count + 1, 0);
-        int64_t lrows = 0, urows = 0, levels = 0;
+        int64_t lrows = 0, urows = 0, levels = 0, entries = 0;
         for (int i = 0; i < count; ++i) {
             const nsg_topology* t = topos[i];
             if (!t) return fail(NSG_ERR_INVALID, "nsg_batch_create: null topology");
@@ -567,12 +612,14 @@ int nsg_batch_create(int count, nsg_topology* const* topos, nsg_batch** out) {
             lrows += (p.lrow_ptr[p.n] + 3) & ~3;
             urows += (p.urow_ptr[p.n] + 3) & ~3;
             levels += static_cast<int64_t>(p.fwd_lev_ptr.size()) - 1;
+            entries += p.nnz_lu - p.n;
             b->a_off[i + 1] = b->a_off[i] + p.nnz_a;
             b->x_off[i + 1] = b->x_off[i] + p.n;
             // keep each instance's LU 32-byte aligned
             b->lu_off[i + 1] = b->lu_off[i] + ((p.nnz_lu + 3) & ~3);
         }
         b->level_rows = static_cast<double>(b->x_off[count]) / std::max<double>(1, levels);
+        b->row_entries = 0.5 * entries / std::max<double>(1, b->x_off[count]);
         // Largest instances first: the grid's tail is made of small ones.
         std::stable_sort(insts.begin(), insts.end(), [&](const nsg::InstDesc& x, const nsg::InstDesc& y) {
             return topos[x.index]->plan.updates > topos[y.index]->plan.updates;
@@ -592,6 +639,7 @@ int nsg_batch_create(int count, nsg_topology* const* topos, nsg_batch** out) {
             (e = upload<double>(&b->d_lrows, nullptr, lrows)) != cudaSuccess ||
             (e = upload<double>(&b->d_urows, nullptr, urows)) != cudaSuccess)
             return cuda_fail("nsg_batch_create", e);
+        create_pool(*b);
         // A plan too large for an update map runs only on the grid-wide
         // schedule (per-warp row maps instead).
         if (b->unmapped) {
@@ -630,8 +678,15 @@ int nsg_batch_solve_complex(nsg_batch* b, const double* d_lu, double* d_x, void*
                        sizeof(double) * 2 * static_cast<size_t>(std::max<long long>(1, b->x_off[b->count])));
         if (e != cudaSuccess) return cuda_fail("nsg_batch_solve_complex: workspace", e);
     }
-    e = nsg::launch_complex_solve(b->d_plans, b->d_pool, b->d_insts, flow_batch(*b), d_lu, d_x,
-                                  b->d_cwork, static_cast<cudaStream_t>(stream));
+    const nsg::FlowBatch fb = flow_batch(*b);
+    const cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (nsg::complex_levels_pay(fb, d_lu)) {
+        StreamScratch w(*b, sizeof(double) * 2 * b->x_off[b->count], st);
+        e = nsg::launch_complex_solve(b->d_plans, b->d_pool, b->d_insts, fb, d_lu, d_x, w.data(), st);
+    } else {
+        e = nsg::launch_complex_solve(b->d_plans, b->d_pool, b->d_insts, fb, d_lu, d_x, b->d_cwork,
+                                      st);
+    }
     return e == cudaSuccess ? NSG_OK : cuda_fail("nsg_batch_solve_complex", e);
 }
 
@@ -707,9 +762,17 @@ int nsg_batch_solve(nsg_batch* b, double* d_x, void* stream) {
 
 int nsg_batch_solve_transposed(nsg_batch* b, double* d_x, void* stream) {
     if (!b || !d_x) return fail(NSG_ERR_INVALID, "nsg_batch_solve_transposed: null argument");
-    cudaError_t e = nsg::launch_solve(b->d_plans, b->d_pool, b->d_insts, flow_batch(*b), b->d_lu,
-                                      d_x, b->d_work, true, nullptr, nullptr,
-                                      static_cast<cudaStream_t>(stream));
+    const nsg::FlowBatch fb = flow_batch(*b);
+    const cudaStream_t st = static_cast<cudaStream_t>(stream);
+    cudaError_t e;
+    if (nsg::transposed_levels_pay(fb)) {
+        StreamScratch w(*b, sizeof(double) * b->x_off[b->count], st);
+        e = nsg::launch_solve(b->d_plans, b->d_pool, b->d_insts, fb, b->d_lu, d_x, w.data(), true,
+                              nullptr, nullptr, st);
+    } else {
+        e = nsg::launch_solve(b->d_plans, b->d_pool, b->d_insts, fb, b->d_lu, d_x, b->d_work, true,
+                              nullptr, nullptr, st);
+    }
     return e == cudaSuccess ? NSG_OK : cuda_fail("nsg_batch_solve_transposed", e);
 }
 

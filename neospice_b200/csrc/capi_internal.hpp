@@ -53,7 +53,11 @@ struct nsg_batch {
     int max_col = 0;
     int max_n = 0;
     double level_rows = 0.0;      // mean rows of a level of the triangular sweeps
+    double row_entries = 0.0;     // mean entries of a row of one
     bool wide = false;            // a plan has wide levels (nsg::wide_levels)
+    // Workspaces of single calls (StreamScratch), kept until the batch is freed;
+    // null where no call of the batch takes one.
+    cudaMemPool_t pool = nullptr;
     bool allow_flow = true;
     int schedule = 0;             // nsg_batch_set_schedule
     int grid_colbuf = 0;          // nsg_batch_set_grid_buffer (0: automatic)
@@ -70,6 +74,7 @@ struct nsg_batch {
     void* d_grid = nullptr;       // flags and state of the grid-wide schedule
     double* d_cwork = nullptr;    // complex sweep workspace (2 doubles per unknown)
     ~nsg_batch() {
+        if (pool) cudaMemPoolDestroy(pool);
         cudaFree(d_rmap);
         cudaFree(d_cwork);
         cudaFree(d_grid);

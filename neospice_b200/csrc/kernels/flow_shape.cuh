@@ -8,11 +8,11 @@
 namespace nsg {
 
 // What the launches depend on: instances, the batch's largest LU column and
-// order, the mean number of rows in a level of its triangular sweeps, and whether
-// any plan has wide levels (wide_levels).
+// order, the mean number of rows in a level of its triangular sweeps and of
+// entries in a row of one, and whether any plan has wide levels (wide_levels).
 struct FlowBatch {
     int count = 0, max_col = 0, max_n = 0;
-    double level_rows = 0.0;
+    double level_rows = 0.0, row_entries = 0.0;
     bool wide = false;
 };
 
@@ -35,6 +35,11 @@ inline int flow_sm_count() {
 // a CTA also takes 1 KB for the system and its static part.
 inline int ctas_per_sm(size_t smem) {
     return static_cast<int>((size_t{228} * 1024) / (smem + 2 * 1024));
+}
+
+// Passes of the SMs over the batch with per_sm CTAs of it on each.
+inline int flow_waves(const FlowBatch& b, int per_sm) {
+    return (b.count + per_sm * flow_sm_count() - 1) / (per_sm * flow_sm_count());
 }
 
 // Levels of fewer rows than this on average: a chain or a band, whose rows wait
@@ -60,6 +65,27 @@ inline FlowShape flow_shape(const FlowBatch& b, size_t many_smem, int need) {
     if (b.count <= flow_sm_count()) return kShapeAlone;
     if (b.count <= 2 * flow_sm_count()) return kShapePair;
     return ctas_per_sm(many_smem) >= need || b.level_rows < kChainRows ? kShapeMany : kShapePair;
+}
+
+// CTAs per SM of the solves that run level after level in global memory (256
+// threads; 48 registers a thread).
+constexpr int kLevelBlocks = 5;
+
+// Whether a transposed or complex solve runs level after level with the vector in
+// a workspace, although the dataflow sweeps, of this shape and with smem bytes a
+// CTA, could keep it in shared memory.  One instance takes R times as long
+// that way, but every SM holds five of them, where shared memory may hold one or
+// two.  R grows with the entries of a row: 1.2 to 1.7 measured for chains and trees
+// (one entry), 2 to 2.5 for a band (6), 4 for a mesh of 577 unknowns (9), 7 of 3137
+// (15), 11 of 16,385 (24).  592 instances, sweeps and levels: chains of 10,000
+// transposed 31.2 and 12.2 ms, complex 32.2 and 14.4; of 3000 complex 5.1 and 3.9;
+// trees of short branches, 10,000 unknowns, 4.6 and 2.5, complex 5.8 and 3.2; meshes
+// of 7057 4.0 and 12.2.  Plans with wide levels keep theirs in shared memory.
+inline bool levels_pay(const FlowBatch& b, FlowShape shape, size_t smem) {
+    if (b.wide) return false;
+    const int fit = ctas_per_sm(smem), most = shape == kShapeMany ? 4 : 2;
+    const int sweeps = flow_waves(b, fit < 1 ? 1 : fit < most ? fit : most);
+    return sweeps > flow_waves(b, kLevelBlocks) * (1.3 + 0.4 * b.row_entries);
 }
 
 }  // namespace nsg

@@ -633,16 +633,24 @@ cudaError_t launch_complex_refactor(const PlanDesc* plans, const int32_t* pool,
     return cudaGetLastError();
 }
 
-// Whether launch_complex_solve keeps the vector in shared memory (and needs no
+// Whether launch_complex_solve can keep the vector in shared memory (and needs no
 // workspace W).
 bool complex_solve_in_smem(int max_n, const double* LU) {
     return complex_sweep_bytes(max_n) <= kMaxCplxSmem && aligned16(LU);
 }
 
+// Whether it had better run level after level in W (2 n doubles per instance) all
+// the same.
+bool complex_levels_pay(const FlowBatch& b, const double* LU) {
+    const size_t smem = complex_sweep_bytes(b.max_n);
+    return complex_solve_in_smem(b.max_n, LU) && levels_pay(b, flow_shape(b, smem, kSolveNeed), smem);
+}
+
+// W null: the dataflow sweeps although the other would pay.
 cudaError_t launch_complex_solve(const PlanDesc* plans, const int32_t* pool, const InstDesc* insts,
                                  const FlowBatch& b, const double* LU, double* X, double* W,
                                  cudaStream_t stream) {
-    if (complex_solve_in_smem(b.max_n, LU)) {
+    if (complex_solve_in_smem(b.max_n, LU) && !(W && complex_levels_pay(b, LU))) {
         const size_t smem = complex_sweep_bytes(b.max_n);
         if (flow_shape(b, smem, kSolveNeed) == kShapeMany)
             return launch_complex(complex_flow_solve_kernel<kWideThreads / 2, 4>, b.count,

@@ -259,13 +259,23 @@ cudaError_t launch_refactor(const PlanDesc* plans, const int32_t* pool, const In
     return cudaGetLastError();
 }
 
+// Whether a transposed solve that could keep its vectors in shared memory had
+// better run level after level in a workspace (n doubles per instance).
+bool transposed_levels_pay(const FlowBatch& b) {
+    const size_t smem = flow_solve_smem_bytes(b.max_n);
+    return smem <= kMaxFlowSmem && levels_pay(b, flow_shape(b, smem, kSolveNeed), smem);
+}
+
+// W: the workspace of a solve level after level; null: the dataflow sweeps although
+// the other would pay.
 cudaError_t launch_solve(const PlanDesc* plans, const int32_t* pool, const InstDesc* insts,
                          const FlowBatch& b, const double* LU, double* X, double* W,
                          bool transposed, const double* lrows, const double* urows,
                          cudaStream_t stream) {
     if (b.count <= 0) return cudaSuccess;
     const size_t smem = flow_solve_smem_bytes(b.max_n);
-    if ((transposed || lrows) && smem <= kMaxFlowSmem) {
+    const bool levels = transposed && W && transposed_levels_pay(b);
+    if ((transposed || lrows) && smem <= kMaxFlowSmem && !levels) {
         const FlowShape shape = flow_shape(b, smem, kSolveNeed);
         const int threads = shape == kShapeMany ? kFlowThreads / 2 : kFlowThreads;
         auto forward = [&](auto kernel) {

@@ -1,6 +1,7 @@
 // Launch shapes of a batch's dataflow kernels without a GPU: the library's own
 // launch functions run against stand-ins for the runtime calls they make.
-// And which plans are solved with a thread per row.  Prints "0 failure(s)" on success.
+// And which plans are solved with a thread per row, which transposed and complex
+// solves run level after level in a workspace.  Prints "0 failure(s)" on success.
 #include "kernels/flow_shape.cuh"
 #include "kernels/lu_device.cuh"
 
@@ -8,6 +9,8 @@
 
 #include <cstdint>
 #include <cstdio>
+#include <set>
+#include <utility>
 
 namespace {
 int threads = 0, failures = 0;
@@ -31,6 +34,8 @@ cudaError_t cudaLaunchKernel(const void*, dim3, dim3 block, void**, size_t, cuda
 
 namespace nsg {
 bool register_wait_limit_setter(cudaError_t (*)(int)) { return true; }
+bool transposed_levels_pay(const FlowBatch&);
+bool complex_levels_pay(const FlowBatch&, const double*);
 cudaError_t launch_refactor(const PlanDesc*, const int32_t*, const InstDesc*, const FlowBatch&,
                             const double*, double*, double, int, double, int32_t*, int32_t*, bool,
                             double*, double*, cudaStream_t);
@@ -83,9 +88,37 @@ void wide(int n, double entries, double level_rows, bool want) {
     }
 }
 
+// the instances of n unknowns with which each solve runs level after level
+void levels(int n, double level_rows, double entries, bool wide, std::set<int> transposed,
+            std::set<int> complex) {
+    for (int count : {1, 148, 149, 296, 297, 592, 740, 741, 1184}) {
+        const nsg::FlowBatch b{count, 32, n, level_rows, entries, wide};
+        if (nsg::transposed_levels_pay(b) != (transposed.count(count) == 1) ||
+            nsg::complex_levels_pay(b, kLu) != (complex.count(count) == 1)) {
+            std::printf("failed: levels of %d, %d instances\n", n, count);
+            ++failures;
+        }
+        // with a workspace the general kernel (256 threads), without one the sweeps
+        double* const w = reinterpret_cast<double*>(64);
+        nsg::launch_complex_solve(nullptr, nullptr, nullptr, b, kLu, nullptr, w, nullptr);
+        if (complex.count(count)) expect("complex levels", n, count, 256);
+        nsg::launch_solve(nullptr, nullptr, nullptr, b, kLu, nullptr, w, true, nullptr, nullptr,
+                          nullptr);
+        if (transposed.count(count)) expect("transposed levels", n, count, 256);
+    }
+}
+
 }  // namespace
 
 int main() {
+    const std::set<int> all = {149, 296, 297, 592, 740, 741, 1184};
+    levels(300, 1.0, 1.0, false, {740}, {740});     // a chain: four CTAs hold 592
+    levels(10000, 1.0, 1.0, false, all, all);       // one CTA
+    levels(10000, 10.0, 1.0, false, all, all);      // a tree of short branches
+    levels(10000, 500.0, 1.0, true, {}, {});        // wide levels
+    levels(9000, 1.0, 6.0, false, {}, {592, 740, 1184});  // a band: two CTAs and one
+    levels(9217, 18.0, 20.0, false, {}, {});        // meshes
+    levels(16385, 21.0, 24.0, false, {}, {});
     // meshes (rows of a level from 2.5 to 20), at the sizes where fewer CTAs fit
     check(37, 12, 2.5, 256, 256, 256, 256);
     check(1601, 96, 10.0, 256, 256, 256, 256);
