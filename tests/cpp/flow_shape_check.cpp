@@ -111,6 +111,11 @@ void levels(int n, double level_rows, double entries, bool wide, std::set<int> t
 }  // namespace
 
 int main() {
+    for (auto [count, want] : {std::pair<int, int>{592, 256}, {700, 512}, {888, 512}, {1184, 256}}) {
+        const nsg::FlowBatch b{count, 64, 577, 7.0, 9.0, false};  // a mesh's last pass
+        nsg::launch_complex_refactor(nullptr, nullptr, nullptr, b, nullptr, kLu, nullptr, nullptr);
+        expect("complex refactor", 577, count, want);
+    }
     const std::set<int> all = {149, 296, 297, 592, 740, 741, 1184};
     levels(300, 1.0, 1.0, false, {740}, {740});     // a chain: four CTAs hold 592
     levels(10000, 1.0, 1.0, false, all, all);       // one CTA
