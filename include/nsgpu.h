@@ -248,7 +248,9 @@ int nsg_batch_refactor_complex(nsg_batch* batch, const double* d_ax, double* d_l
  * holds b on entry and x on return, interleaved, 2*vector_offsets per
  * instance.  The vectors are kept in shared memory up to 10,240 unknowns and for
  * a d_lu that is 16-byte aligned; else the first call allocates the batch's
- * complex sweep workspace. */
+ * complex sweep workspace.  (Large batches of long chains take a workspace for
+ * the time of a call, here and in nsg_batch_solve_transposed, from a pool that
+ * the batch keeps until it is freed; not while the stream is captured.) */
 int nsg_batch_solve_complex(nsg_batch* batch, const double* d_lu, double* d_x, void* stream);
 
 /* Device pointer to the factored LU values (layout per nsg_batch_layout and
